@@ -58,8 +58,9 @@ namespace cpt {
 cpt_status wavefront_grids(int sm_count, int block_trace, int block_shade, int short_entries, int* grid_trace,
                            int* grid_trace_wide, int* grid_shade);
 size_t wide_scratch_bytes(uint32_t n);
-cpt_status build_wide(uint32_t n, const int2* child, const float4* node_box, const float4* leaf_box, float4* wide,
-                      void* scratch, size_t scratch_bytes, cudaStream_t stream, uint32_t* num_wide);
+cpt_status build_wide(uint32_t n, const int2* child, const float4* node_box, const float4* leaf_box,
+                      const uint32_t* order, float4* wide, void* scratch, size_t scratch_bytes, cudaStream_t stream,
+                      uint32_t* num_wide, const uint32_t** wide_order);
 }
 
 struct cpt_scene {
@@ -446,12 +447,12 @@ cpt_status make_layout(cpt_scene* s, cudaStream_t stream, uint32_t* num_wide)
         }
         if (wide_scratch_bytes(n) > s->scratch_bytes) return fail(CPT_ERR_INVALID_ARGUMENT, "wide scratch too small");
         s->width = 8;
-        // leaf records in sorted (Morton) order, shared with the binary layout
-        cpt_status st = build_trace_layout(n, s->n_lights, s->n_spheres, s->child, s->node_box, s->leaf_box, s->order,
-                                           s->tri_f32, s->tri_f64, s->spheres, nullptr, s->leaf_rec, stream);
+        const uint32_t* wide_order = nullptr;   // primitives of the leaves in the wide layout's order
+        cpt_status st = build_wide(n, s->child, s->node_box, s->leaf_box, s->order, s->wide, s->scratch,
+                                   s->scratch_bytes, stream, num_wide, &wide_order);
         if (st != CPT_OK) return st;
-        return build_wide(n, s->child, s->node_box, s->leaf_box, s->wide, s->scratch, s->scratch_bytes, stream,
-                          num_wide);
+        return build_trace_layout(n, s->n_lights, s->n_spheres, s->child, s->node_box, s->leaf_box, wide_order,
+                                  s->tri_f32, s->tri_f64, s->spheres, nullptr, s->leaf_rec, stream);
     }
     if (!s->nodes && ni) {
         cpt_status st = dalloc(&s->nodes, 4 * (size_t)ni);

@@ -10,7 +10,6 @@
 #define CPT_STACK 64                          // Karras trees over 64-bit keys are at most 65 levels deep
 #define CPT_WSTACK 72                         // 8-wide traversal: at most one node group per level
 #define CPT_WIDE_F4 6                         // float4 per wide node (96 bytes)
-#define CPT_WIDE_EMPTY 0x7fffffff             // child reference of an unused wide-node slot
 
 // Primitive kinds stored in leaf records (w of the second float4).
 enum { CPT_KIND_TRI = 0, CPT_KIND_SPHERE = 1, CPT_KIND_LIGHT = 2 };

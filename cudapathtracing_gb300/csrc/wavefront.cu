@@ -328,7 +328,8 @@ __global__ void k_wf_finish(JobGeo jg, RenderArgs a, int groups)
 
 // BVH2: at most 48 registers (5 blocks of 256 per SM): 62 % occupancy instead of 50 % for a few
 // spilled values, +5.7 % on the 1080p spheres render (the shadow kernel is faster uncapped).
-// 8-wide: at most 64 registers (4 blocks of 256): +4.7 % against 72; 51 registers spill (-9 %).
+// 8-wide: at most 64 registers (4 blocks of 256): 283 ms for the 64-spp 1080p frame, 293 ms at 48
+// or 80 registers.
 template <bool WIDE, int SHORT, bool SORT, bool MULTI>
 __global__ void __launch_bounds__(256, WIDE ? 4 : 5) k_wf_trace(const __grid_constant__ SceneView s, Wf w, int par)
 {
@@ -382,8 +383,9 @@ __global__ void __launch_bounds__(256, WIDE ? 4 : 5) k_wf_trace(const __grid_con
     count_rays(w.rays, rays);
 }
 
+// 64 registers (4 blocks of 256), as the 8-wide extension-ray kernel (48: +4 % time, 80: +4 %).
 template <bool WIDE, int SHORT, bool MULTI>
-__global__ void __launch_bounds__(256) k_wf_shadow(const __grid_constant__ SceneView s, Wf w, int par)
+__global__ void __launch_bounds__(256, 4) k_wf_shadow(const __grid_constant__ SceneView s, Wf w, int par)
 {
     const int n = w.cnt[4 + par];
     const int* sq = w.sq + (size_t)par * w.M * w.L;

@@ -14,12 +14,16 @@
 // octant o meets the children roughly in the order of slots s ^ (7 ^ o) — the ordering scheme of
 // compressed wide BVHs (Ylitie, Karras, Laine 2017), which needs no sort during traversal.
 //
-// Node layout (96 bytes, six 16-byte loads):
-//   float4 f0   origin p.xyz (node box minimum); w = ex | ey << 8 | ez << 16 | imask << 24
-//               (biased grid exponents; bit s of imask: slot s holds an internal child)
-//   int4 f1,f2  child reference of slots 0..7: >= 0 wide (= binary) node, < 0 leaf ~k,
-//               CPT_WIDE_EMPTY for an unused slot
-//   f3,f4,f5    8-bit quantised child boxes: (lo slots 0-3, lo 4-7, hi 0-3, hi 4-7) for x, y, z
+// Node layout (96 bytes, three 32-byte loads; i and l are the node's internal and leaf children):
+//   float4 f0   origin p.xyz (node box minimum), grid step of x
+//   f1          grid steps of y and z; number of the first internal child; index of the first leaf
+//   f2,f3,f4    8-bit quantised child boxes: (lo slots 0-3, lo 4-7, hi 0-3, hi 4-7) for x, y, z
+//   f5          x: mask of the internal slots | mask of the leaf slots << 8, slot s at bit 7 - s
+// A node's internal children have consecutive numbers and its leaves consecutive leaf records, both
+// in slot order, so a child's reference is the first one plus a population count.  Leaf records are
+// therefore stored in this layout's own order: the leaves of a node share memory sectors, and the
+// 32 bytes that eight references would take hold the grid steps, which the traversal would
+// otherwise decode from exponents on every visit.
 //
 // Child boxes sit on a power-of-two grid anchored at p with 255 steps across the node, rounded
 // outwards, so every quantised box contains the child's FP32 box.
@@ -63,6 +67,9 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS, 3) k_collapse_level(const in
                                                                      int* __restrict__ tasks,
                                                                      int* __restrict__ level_count,
                                                                      int* __restrict__ level_base, int l,
+                                                                     const uint32_t* __restrict__ order,
+                                                                     uint32_t* __restrict__ wide_order,
+                                                                     uint32_t* __restrict__ n_leaves,
                                                                      float4* __restrict__ wide)
 {
     const int n = level_count[l];
@@ -79,7 +86,7 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS, 3) k_collapse_level(const in
         ref_box(b, node_box, leaf_box, nmn, nmx);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-            refs[k] = CPT_WIDE_EMPTY;
+            refs[k] = -1;
             car[k] = -1.0f;
         }
         refs[0] = c.x;
@@ -159,36 +166,29 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS, 3) k_collapse_level(const in
                 if (k == bk) slot_of[k] = bs;
             used |= 1u << bs;
         }
-        // Internal children take consecutive wide numbers in slot order: the child in slot s is
-        // number first_child + (internal children in slots below s).
-        uint32_t imask = 0;
+        // Internal children take consecutive wide numbers and leaves consecutive records, both in
+        // slot order: the child in slot s is number first + (children of its kind in slots below s).
+        uint32_t imask = 0, lmask = 0;   // slot s at bit 7 - s
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-            if (k < nr && refs[k] >= 0) imask |= 1u << slot_of[k];
-        const int n_int = __popc(imask);
-        const int first_child = n_int ? atomicAdd(n_out, n_int) : 0;
+            if (k < nr) (refs[k] >= 0 ? imask : lmask) |= 0x80u >> slot_of[k];
+        const int n_int = __popc(imask), n_leaf = __popc(lmask);
+        const int first_child = base + n + (n_int ? atomicAdd(n_out, n_int) : 0);
+        const uint32_t first_leaf = n_leaf ? atomicAdd(n_leaves, (uint32_t)n_leaf) : 0u;
         const uint32_t ex = grid_exponent(nmn.x, nmx.x), ey = grid_exponent(nmn.y, nmx.y),
                        ez = grid_exponent(nmn.z, nmx.z);
         const float isx = inv_grid(ex), isy = inv_grid(ey), isz = inv_grid(ez);
         uint32_t q[6][2];
 #pragma unroll
         for (int a = 0; a < 6; ++a) q[a][0] = q[a][1] = 0;
-        int at_slot[8];
-#pragma unroll
-        for (int s2 = 0; s2 < 8; ++s2) at_slot[s2] = CPT_WIDE_EMPTY;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             if (k >= nr) break;
             const int s = slot_of[k];
-            int ref = refs[k];
-            if (ref >= 0) {
-                const int num = first_child + __popc(imask & ((1u << s) - 1u));
-                ref = base + n + num;   // the child's wide node number
-                tasks[ref] = refs[k];
-            }
-#pragma unroll
-            for (int s2 = 0; s2 < 8; ++s2)
-                if (s2 == s) at_slot[s2] = ref;
+            if (refs[k] >= 0)
+                tasks[first_child + __popc(imask >> (8 - s))] = refs[k];
+            else
+                wide_order[first_leaf + __popc(lmask >> (8 - s))] = order[~refs[k]];
             const uint32_t sh = (uint32_t)(s & 3) * 8u;
             const uint32_t v[6] = {q_lo(cmn[k].x, nmn.x, isx) << sh, q_hi(cmx[k].x, nmn.x, isx) << sh,
                                    q_lo(cmn[k].y, nmn.y, isy) << sh, q_hi(cmx[k].y, nmn.y, isy) << sh,
@@ -202,37 +202,41 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS, 3) k_collapse_level(const in
             }
         }
         float4* dst = wide + CPT_WIDE_F4 * (size_t)(base + t);
-        dst[0] = make_float4(nmn.x, nmn.y, nmn.z, __int_as_float((int)(ex | (ey << 8) | (ez << 16) | (imask << 24))));
-        dst[1] = make_float4(__int_as_float(at_slot[0]), __int_as_float(at_slot[1]), __int_as_float(at_slot[2]),
-                             __int_as_float(at_slot[3]));
-        dst[2] = make_float4(__int_as_float(at_slot[4]), __int_as_float(at_slot[5]), __int_as_float(at_slot[6]),
-                             __int_as_float(at_slot[7]));
+        dst[0] = make_float4(nmn.x, nmn.y, nmn.z, __uint_as_float(ex << 23));
+        dst[1] = make_float4(__uint_as_float(ey << 23), __uint_as_float(ez << 23), __int_as_float(first_child),
+                             __uint_as_float(first_leaf));
 #pragma unroll
         for (int a = 0; a < 3; ++a)
-            dst[3 + a] = make_float4(__int_as_float((int)q[2 * a][0]), __int_as_float((int)q[2 * a][1]),
+            dst[2 + a] = make_float4(__int_as_float((int)q[2 * a][0]), __int_as_float((int)q[2 * a][1]),
                                      __int_as_float((int)q[2 * a + 1][0]), __int_as_float((int)q[2 * a + 1][1]));
+        dst[5] = make_float4(__uint_as_float(imask | lmask << 8), 0.f, 0.f, 0.f);
     }
 }
 
-__global__ void k_collapse_init(int* tasks, int* level_count, int* level_base)
+__global__ void k_collapse_init(int* tasks, int* level_count, int* level_base, uint32_t* n_leaves)
 {
     for (int i = threadIdx.x; i < MAX_WIDE_LEVELS; i += blockDim.x) {
         level_count[i] = i == 0 ? 1 : 0;   // level 0: the root
         level_base[i] = 0;
     }
-    if (threadIdx.x == 0) tasks[0] = 0;   // wide node 0 stands for the binary root
+    if (threadIdx.x == 0) {
+        tasks[0] = 0;   // wide node 0 stands for the binary root
+        *n_leaves = 0;
+    }
 }
 
 }  // namespace
 
 size_t wide_scratch_bytes(uint32_t n)
 {
-    // the binary node of every wide node (at most n - 1 of them), and the level counts and bases
-    return align_up((size_t)n * 4, 256) + align_up(2 * MAX_WIDE_LEVELS * 4, 256);
+    // the binary node of every wide node (at most n - 1 of them), the leaves' primitives in the
+    // wide layout's order, and the level counts and bases and the leaf count
+    return 2 * align_up((size_t)n * 4, 256) + align_up((2 * MAX_WIDE_LEVELS + 1) * 4, 256);
 }
 
-cpt_status build_wide(uint32_t n, const int2* child, const float4* node_box, const float4* leaf_box, float4* wide,
-                      void* scratch, size_t scratch_bytes, cudaStream_t stream, uint32_t* num_wide)
+cpt_status build_wide(uint32_t n, const int2* child, const float4* node_box, const float4* leaf_box,
+                      const uint32_t* order, float4* wide, void* scratch, size_t scratch_bytes, cudaStream_t stream,
+                      uint32_t* num_wide, const uint32_t** wide_order)
 {
     if (n < 2) {
         if (num_wide) *num_wide = 0;
@@ -242,9 +246,13 @@ cpt_status build_wide(uint32_t n, const int2* child, const float4* node_box, con
     char* p = (char*)scratch;
     int* tasks = (int*)p;
     p += align_up((size_t)n * 4, 256);
+    uint32_t* prims = (uint32_t*)p;
+    *wide_order = prims;
+    p += align_up((size_t)n * 4, 256);
     int* level_count = (int*)p;
     int* level_base = level_count + MAX_WIDE_LEVELS;
-    k_collapse_init<<<1, 128, 0, stream>>>(tasks, level_count, level_base);
+    uint32_t* n_leaves = (uint32_t*)(level_base + MAX_WIDE_LEVELS);
+    k_collapse_init<<<1, 128, 0, stream>>>(tasks, level_count, level_base, n_leaves);
     add_launches(1);
     // A grid that is resident at once; each thread takes nodes of its level in turn.  The host
     // looks at the level counts once every 16 levels (the wide tree of a few million primitives
@@ -268,7 +276,7 @@ cpt_status build_wide(uint32_t n, const int2* child, const float4* node_box, con
         const int first = l, stop = std::min(l + 16, MAX_WIDE_LEVELS - 1);
         for (; l < stop; ++l)
             k_collapse_level<<<grid, COLLAPSE_THREADS, 0, stream>>>(child, node_box, leaf_box, tasks, level_count,
-                                                                    level_base, l, wide);
+                                                                    level_base, l, order, prims, n_leaves, wide);
         add_launches(stop - first);
         CPT_CUDA(cudaGetLastError());
         // level l: its count (wide nodes still to collapse) and base (= wide nodes written)
