@@ -100,6 +100,7 @@ struct WavefrontTuning {
     int grid_trace, block_trace; // persistent grids (grid_trace_wide: the 8-wide trace kernels)
     int grid_trace_wide;
     int grid_shade, block_shade;
+    int grid_paths;              // persistent grid of the kernel that finishes a render's last paths
     int short_stack;             // traversal stack entries kept in shared memory (8, 16, 24, 32)
     bool use_graph;
     bool material_sort;          // shade slots binned by the material their ray hit

@@ -278,6 +278,11 @@ __device__ __forceinline__ void sample_ggx_reflect(const Surf& sf, float3 ray_d,
 
 // Material::sampleLight (Material.cuh:95-193) + cosine-weighted Lambertian (the reference's
 // commented sampler, Material.cuh:177-188).  Writes sf.wm for the rough dielectric.
+//
+// PINNED (the wavefront, whose kernels must shade a vertex to the same bits) spells out the
+// multiply-adds of the mirror direction's dot product: left to the compiler, one kernel takes it from
+// the Fresnel term's (a rounding apart) and another computes it.
+template <bool PINNED = false>
 __device__ __forceinline__ void bsdf_sample(Surf& sf, float3 ray_d, float3& dir, float& pdf, float r1, float r2, float r3)
 {
     const float3 n = sf.normal;
@@ -286,7 +291,8 @@ __device__ __forceinline__ void bsdf_sample(Surf& sf, float3 ray_d, float3& dir,
         float3 urd = unit3(ray_d);
         float R = fresnel_dielectric(n, -urd, rr);
         if (r3 < R) {
-            dir = urd - 2.0f * dot3(urd, n) * n;
+            const float un = PINNED ? __fmaf_rn(urd.z, n.z, __fmaf_rn(urd.x, n.x, __fmul_rn(urd.y, n.y))) : dot3(urd, n);
+            dir = urd - 2.0f * un * n;
             pdf = R;
         } else {
             float3 vperp = (1.0f / rr) * (urd + dot3(-urd, n) * n);

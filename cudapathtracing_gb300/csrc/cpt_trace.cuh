@@ -66,8 +66,10 @@ __device__ __forceinline__ bool hit_light(const DevLight& L, float3 o, float3 d,
     return fabsf(u) <= L.w / 2.0f && fabsf(v) <= L.h / 2.0f;
 }
 
+// Hit of leaf k in [0.001, tmax]; with SKIP the light `skip` is never hit.
+template <bool SKIP = false>
 __device__ __forceinline__ bool hit_leaf(const SceneView& s, int k, float3 o, float3 d, float tmax, float& t, float& u,
-                                         float& v)
+                                         float& v, int skip = -1)
 {
     const float4* r = s.leaf_rec + 3 * (size_t)k;
     float4 r0 = ldg4(r), r1 = ldg4(r + 1);
@@ -79,7 +81,8 @@ __device__ __forceinline__ bool hit_leaf(const SceneView& s, int k, float3 o, fl
     }
     u = v = 0.f;
     if (kind == CPT_KIND_SPHERE) return hit_sphere(o, d, f3(r0.x, r0.y, r0.z), r1.x, 0.001f, tmax, t);
-    return hit_light(s.lights[__float_as_int(r1.x)], o, d, 0.001f, tmax, t);
+    const int li = __float_as_int(r1.x);
+    return (!SKIP || li != skip) && hit_light(s.lights[li], o, d, 0.001f, tmax, t);
 }
 
 // Occlusion test of leaf k for a shadow ray aimed at light `skip`: any primitive hit in
@@ -100,20 +103,24 @@ __device__ __forceinline__ bool occludes_leaf(const SceneView& s, int k, float3 
     return li != skip && hit_light(s.lights[li], o, d, 0.001f, tmax, t);
 }
 
-// One leaf reached by a traversal.  Closest-hit queries (ANY false) keep the nearest hit in
-// [0.001, best]; occlusion queries (ANY true) return true at the first occluder.
-template <bool ANY>
+// What a traversal asks: the closest hit, any occluder of a shadow ray, or either, per ray.
+enum Query { Q_CLOSEST, Q_ANY, Q_EITHER };
+
+// One leaf reached by a traversal.  Closest-hit queries keep the nearest hit in [0.001, best];
+// occlusion queries (Q_ANY, or Q_EITHER with any set) return true at the first occluder.
+template <Query Q>
 __device__ __forceinline__ bool visit_leaf(const SceneView& s, int leaf, float3 o, float3 d, float& best, Hit& hit,
-                                           int skip)
+                                           int skip, bool any)
 {
-    if (ANY) {
+    if (Q == Q_ANY) {
         if (!occludes_leaf(s, leaf, o, d, best, skip)) return false;
         hit.leaf = leaf;
         return true;
     }
     float t, u, v;
-    if (hit_leaf(s, leaf, o, d, best, t, u, v)) {
+    if (hit_leaf<Q == Q_EITHER>(s, leaf, o, d, best, t, u, v, skip)) {
         best = t; hit.t = t; hit.u = u; hit.v = v; hit.leaf = leaf;
+        return Q == Q_EITHER && any;
     }
     return false;
 }
@@ -191,8 +198,8 @@ __device__ __forceinline__ uint32_t xor_bits(uint32_t v, uint32_t o)
 // internal child and keeps the rest as one node-group entry (first child's number, node's internal
 // mask, remaining hit bits) on the stack, as in compressed wide BVH traversal (Ylitie et al. 2017);
 // a popped group yields its next child without touching memory.  Boxes are tested against the
-// closest hit so far, so far subtrees are culled.  With ANY the walk is an occlusion query
-// (visit_leaf) that stops at the first occluder.  The walk advances one node per step() so that a
+// closest hit so far, so far subtrees are culled.  An occlusion query (visit_leaf) stops at the
+// first occluder.  The walk advances one node per step() so that a
 // warp can refill finished lanes (dynamic fetching); Stack64 keeps group entries (in shared and
 // local memory, or local only).
 //
@@ -205,16 +212,17 @@ __device__ __forceinline__ uint32_t xor_bits(uint32_t v, uint32_t o)
 // scalar multiply-adds, 283 ms packed.  Measured and left out: prefetching the next node before the
 // leaf tests (+4 %), testing the three interval conditions by sign instead of min/max with tmin and
 // best (+2 %).
-template <bool ANY, typename Stack64>
+template <Query Q, typename Stack64>
 struct WideWalk {
     float3 o, d, idir;
     float tmin, best;
     uint32_t first, node;
     int sp, skip;
+    bool any;   // Q_EITHER: this ray asks for any occluder
     Hit hit;
     Stack64 stack;
 
-    __device__ __forceinline__ void start(float3 o_, float3 d_, float tmin_, float tmax_, int skip_)
+    __device__ __forceinline__ void start(float3 o_, float3 d_, float tmin_, float tmax_, int skip_, bool any_ = false)
     {
         o = o_;
         d = d_;
@@ -225,6 +233,7 @@ struct WideWalk {
         node = 0;
         sp = 0;
         skip = skip_;
+        any = any_;
         hit.leaf = -1;
         hit.t = tmax_;
         hit.u = hit.v = 0.f;
@@ -319,7 +328,7 @@ struct WideWalk {
         while (lhits) {
             const uint32_t slot = (uint32_t)(__ffs(lhits) - 1) ^ first;
             lhits &= lhits - 1;
-            if (visit_leaf<ANY>(s, (int)(leaf0 + __popc(lmask >> (8u - slot))), o, d, best, hit, skip)) return true;
+            if (visit_leaf<Q>(s, (int)(leaf0 + __popc(lmask >> (8u - slot))), o, d, best, hit, skip, any)) return true;
         }
         return done;
     }
@@ -359,7 +368,7 @@ template <bool ANY>
 __device__ __forceinline__ bool trace_closest_wide(const SceneView& s, float3 o, float3 d, float tmin, float tmax,
                                                    Hit& hit, int* err, int skip)
 {
-    WideWalk<ANY, LocalStack64> w;
+    WideWalk<ANY ? Q_ANY : Q_CLOSEST, LocalStack64> w;
     w.stack.init();
     w.start(o, d, tmin, tmax, skip);
     while (!w.step(s, err)) {}
@@ -436,8 +445,8 @@ __device__ __forceinline__ bool trace_closest_bvh2(const SceneView& s, float3 o,
         float bf = fminf(fminf(fmaxf(r.bx0, r.bx1), fmaxf(r.by0, r.by1)), fminf(fmaxf(r.bz0, r.bz1), best));
         int ca = r.ca, cb = r.cb;
         bool ha = an <= af, hb = bn <= bf;
-        if (ha && ca < 0 && visit_leaf<ANY>(s, ~ca, o, d, best, hit, skip)) return true;
-        if (hb && cb < 0 && visit_leaf<ANY>(s, ~cb, o, d, best, hit, skip)) return true;
+        if (ha && ca < 0 && visit_leaf<ANY ? Q_ANY : Q_CLOSEST>(s, ~ca, o, d, best, hit, skip, ANY)) return true;
+        if (hb && cb < 0 && visit_leaf<ANY ? Q_ANY : Q_CLOSEST>(s, ~cb, o, d, best, hit, skip, ANY)) return true;
         bool ta = ha && ca >= 0, tb = hb && cb >= 0;
         if (ta && tb) {
             bool anear = an <= bn;
@@ -463,15 +472,16 @@ __device__ __forceinline__ bool trace_closest_bvh2(const SceneView& s, float3 o,
 // One ray's traversal state, advanced one node per call, so that a warp can refill lanes whose
 // ray finished with new rays instead of waiting for its slowest lane (dynamic ray fetching,
 // Aila & Laine 2009).  The visit order and pruning are those of trace_closest_bvh2.
-template <bool ANY, typename Stack>
+template <Query Q, typename Stack>
 struct Bvh2Walk {
     float3 o, d, idir, ood;
     float tmin, best;
     int node, sp, skip;
+    bool any;   // Q_EITHER: this ray asks for any occluder
     Hit hit;
     Stack stack;   // init() once per kernel, before the first start()
 
-    __device__ __forceinline__ void start(float3 o_, float3 d_, float tmin_, float tmax_, int skip_)
+    __device__ __forceinline__ void start(float3 o_, float3 d_, float tmin_, float tmax_, int skip_, bool any_ = false)
     {
         o = o_;
         d = d_;
@@ -482,6 +492,7 @@ struct Bvh2Walk {
         node = 0;
         sp = 0;
         skip = skip_;
+        any = any_;
         hit.leaf = -1;
         hit.t = tmax_;
         hit.u = hit.v = 0.f;
@@ -498,8 +509,8 @@ struct Bvh2Walk {
         float bf = fminf(fminf(fmaxf(r.bx0, r.bx1), fmaxf(r.by0, r.by1)), fminf(fmaxf(r.bz0, r.bz1), best));
         int ca = r.ca, cb = r.cb;
         bool ha = an <= af, hb = bn <= bf;
-        if (ha && ca < 0 && visit_leaf<ANY>(s, ~ca, o, d, best, hit, skip)) return true;
-        if (hb && cb < 0 && visit_leaf<ANY>(s, ~cb, o, d, best, hit, skip)) return true;
+        if (ha && ca < 0 && visit_leaf<Q>(s, ~ca, o, d, best, hit, skip, any)) return true;
+        if (hb && cb < 0 && visit_leaf<Q>(s, ~cb, o, d, best, hit, skip, any)) return true;
         bool ta = ha && ca >= 0, tb = hb && cb >= 0;
         if (ta && tb) {
             bool anear = an <= bn;
@@ -583,7 +594,7 @@ template <bool ANY, typename Stack, typename Views, typename Load, typename Stor
 __device__ __forceinline__ uint32_t trace_items_bvh2_views(const Views& views, int n, int* fetch, int* err, Load load,
                                                            Store store)
 {
-    return trace_items_walk<Bvh2Walk<ANY, Stack>>(views, n, fetch, err, load, store);
+    return trace_items_walk<Bvh2Walk<ANY ? Q_ANY : Q_CLOSEST, Stack>>(views, n, fetch, err, load, store);
 }
 
 // Dynamic fetching over the 8-wide BVH (the same refill policy).
@@ -591,7 +602,7 @@ template <bool ANY, typename Stack64, typename Views, typename Load, typename St
 __device__ __forceinline__ uint32_t trace_items_wide_views(const Views& views, int n, int* fetch, int* err, Load load,
                                                            Store store)
 {
-    return trace_items_walk<WideWalk<ANY, Stack64>>(views, n, fetch, err, load, store);
+    return trace_items_walk<WideWalk<ANY ? Q_ANY : Q_CLOSEST, Stack64>>(views, n, fetch, err, load, store);
 }
 
 // The same over one scene.
@@ -620,7 +631,7 @@ __device__ __forceinline__ bool trace_closest(const SceneView& s, float3 o, floa
     if (s.n_prims <= 0) return false;
     if (s.n_internal == 0) {
         float best = tmax;
-        visit_leaf<ANY>(s, 0, o, d, best, hit, skip);
+        visit_leaf<ANY ? Q_ANY : Q_CLOSEST>(s, 0, o, d, best, hit, skip, ANY);
         return hit.leaf >= 0;
     }
     if (WIDE) return trace_closest_wide<ANY>(s, o, d, tmin, tmax, hit, err, skip);

@@ -70,11 +70,14 @@ def poisson_jobs(n: int, rate: float = 20.0, seed: int = 3, denoise_frac: float 
 def job_bytes(num_triangles: int, size: int, spp: int, slots: int = 1 << 21) -> int:
     """Device memory of one job: triangles, BVH nodes and leaf records, build scratch (~300 B per
     triangle), the image, G-buffer and denoiser activations (~700 B per pixel), and the wavefront
-    state (slots and per-item group sums)."""
+    state (slots and per-item sums; a small render's items are single samples, with G-buffer entries
+    beside their sums)."""
     px = size * size
     groups = max(1, (spp + 7) // 8)
-    items = px * groups
-    return int(300 * num_triangles + 700 * px + 200 * min(slots, items) + 16 * items)
+    items, per_item = px * groups, 16
+    if items <= 1 << 21 and px * spp <= 1 << 24:
+        items, per_item = px * spp, 48
+    return int(300 * num_triangles + 700 * px + 200 * min(slots, items) + per_item * items)
 
 
 class Scheduler:
