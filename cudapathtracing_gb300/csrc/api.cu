@@ -43,6 +43,12 @@ void ini_free(IniScene* s);
 
 using namespace cpt;
 
+struct HostWords {
+    unsigned long long rays;
+    int err;
+    int cnt[16];
+};
+
 struct cpt_context {
     int device;
     int sm_count;
@@ -52,7 +58,22 @@ struct cpt_context {
     int bvh_width;             // traversal layout built by cpt_lbvh_build: 8 (compressed wide) or 2
     int iter_limit;            // loop trips per sample of the render loops (cpt_context_set_loop_limits)
     bool bvh2_compressed;      // BVH2 nodes of later builds: 32-byte quantised (cpt_context_set_bvh_compression)
+    // Workspaces of the calls (path slots, filter and host-image buffers) come from a pool of the
+    // context's own that keeps up to pool_keep bytes between calls and goes with the context.  The
+    // device's default pool gives everything back to the system whenever a stream is waited for, and
+    // every call waits: 0.33 ms per call for a 256 x 256 preview's slots, 0.2 ms for a 1080p filter.
+    cudaMemPool_t pool;        // NULL until need_pool
+    HostWords* host;           // pinned words that results are read back into, or NULL (need_host)
+    char* staging;             // pinned and mapped: rays and hits of small host-memory queries, or NULL
+    char* staging_dev;         // its device address
+    int trace_resident[2];     // blocks of the trace kernels that fit at once (0: not queried yet)
+    cudaEvent_t time[6];       // timing events of the calls that report device times
 };
+
+// Small queries on host memory (picking, probes) are read and answered in place: the kernel reads
+// the rays from pinned memory and writes the hits there, which saves both copies and both
+// allocations (1,000 rays: 244 us with them).  Larger ones are copied.
+constexpr uint64_t STAGED_RAYS = 16384;
 
 namespace cpt {
 cpt_status wavefront_grids(int sm_count, int block_trace, int block_shade, int short_entries, int* grid_trace,
@@ -477,12 +498,60 @@ LbvhBuffers buffers_of(cpt_scene* s)
     return b;
 }
 
+// The context's workspace pool, made by the first call that needs it.
+cpt_status need_pool(cpt_context* c)
+{
+    if (c->pool) return CPT_OK;
+    cudaMemPoolProps props;
+    std::memset(&props, 0, sizeof props);
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = c->device;
+    size_t free_bytes = 0, total_bytes = 0;
+    CPT_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+    uint64_t keep = total_bytes / 40;   // 7 GB of 284: the largest wavefront (16M slots) takes 5.4
+    cudaMemPool_t pool = nullptr;
+    CPT_CUDA(cudaMemPoolCreate(&pool, &props));
+    cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+        cudaMemPoolDestroy(pool);
+        return cuda_fail(e, "workspace pool");
+    }
+    c->pool = c->wf.pool = pool;
+    return CPT_OK;
+}
+
+// The context's pinned words and timing events, made by the first call that reads a result back.
+cpt_status need_host(cpt_context* c)
+{
+    if (c->host) return CPT_OK;
+    HostWords* h = nullptr;
+    CPT_CUDA(cudaMallocHost((void**)&h, sizeof(HostWords)));
+    for (int i = 0; i < (int)(sizeof c->time / sizeof c->time[0]); ++i) {
+        cudaError_t e = cudaEventCreate(&c->time[i]);
+        if (e != cudaSuccess) {
+            while (i--) cudaEventDestroy(c->time[i]);
+            cudaFreeHost(h);
+            return cuda_fail(e, "timing events");
+        }
+    }
+    c->host = h;
+    c->wf.host_cnt = h->cnt;
+    return CPT_OK;
+}
+
+#define CPT_NEED(call)                      \
+    do {                                    \
+        cpt_status _s = (call);             \
+        if (_s != CPT_OK) return _s;        \
+    } while (0)
+
 // Reads and clears the device error word (synchronises the stream).
 cpt_status check_device_error(cpt_scene* s, cudaStream_t stream)
 {
-    int e = 0;
-    CPT_CUDA(cudaMemcpyAsync(&e, s->err, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    CPT_CUDA(cudaMemcpyAsync(&s->ctx->host->err, s->err, sizeof(int), cudaMemcpyDeviceToHost, stream));
     CPT_CUDA(cudaStreamSynchronize(stream));
+    const int e = s->ctx->host->err;
     if (e) {
         CPT_CUDA(cudaMemsetAsync(s->err, 0, sizeof(int), stream));
         if (e & CPT_DEVERR_STACK) return fail(CPT_ERR_STACK_OVERFLOW, "traversal stack limit exceeded");
@@ -532,6 +601,10 @@ CPT_EXPORT cpt_status cpt_context_create(int device, cpt_context** out)
     CPT_CUDA(cudaStreamCreateWithFlags(&c->wf.side_stream, cudaStreamNonBlocking));
     CPT_CUDA(cudaEventCreateWithFlags(&c->wf.fork, cudaEventDisableTiming));
     CPT_CUDA(cudaEventCreateWithFlags(&c->wf.join, cudaEventDisableTiming));
+    c->pool = nullptr;
+    c->host = nullptr;
+    c->staging = c->staging_dev = nullptr;
+    c->trace_resident[0] = c->trace_resident[1] = 0;
     *out = c;
     return CPT_OK;
 }
@@ -542,6 +615,14 @@ CPT_EXPORT cpt_status cpt_context_destroy(cpt_context* ctx)
     if (ctx && ctx->wf.side_stream) cudaStreamDestroy(ctx->wf.side_stream);
     if (ctx && ctx->wf.fork) cudaEventDestroy(ctx->wf.fork);
     if (ctx && ctx->wf.join) cudaEventDestroy(ctx->wf.join);
+    if (ctx) {
+        if (ctx->host) {
+            for (cudaEvent_t e : ctx->time) cudaEventDestroy(e);
+            cudaFreeHost(ctx->host);
+        }
+        if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
+        if (ctx->staging) cudaFreeHost(ctx->staging);
+    }
     delete ctx;
     return CPT_OK;
 }
@@ -601,7 +682,8 @@ CPT_EXPORT cpt_status cpt_filter_bilateral(cpt_context* ctx, const float* rgb, c
     if (params) p = *params;
     if (rgb == out) return fail(CPT_ERR_INVALID_ARGUMENT, "cpt_filter_bilateral: out must not alias rgb");
     CPT_CUDA(cudaSetDevice(ctx->device));
-    return filter_bilateral(rgb, gbuf, out, width, height, p, (cudaStream_t)stream);
+    CPT_NEED(need_pool(ctx));
+    return filter_bilateral(rgb, gbuf, out, width, height, p, (cudaStream_t)stream, ctx->pool);
 }
 
 CPT_EXPORT cpt_status cpt_filter_temporal(cpt_context* ctx, float* rgb, const float* prev_rgb, const float* gbuf,
@@ -703,35 +785,29 @@ CPT_EXPORT cpt_status cpt_lbvh_build(cpt_scene* s, void* stream_, cpt_bvh_stats*
     if (!s) return fail(CPT_ERR_INVALID_ARGUMENT, "cpt_lbvh_build: scene is NULL");
     cudaStream_t stream = (cudaStream_t)stream_;
     CPT_CUDA(cudaSetDevice(s->ctx->device));
-    LbvhTimings tm = {0, 0, 0, 0};
-    cudaEvent_t e0, e1;
-    if (stats) {
-        CPT_CUDA(cudaEventCreate(&e0));
-        CPT_CUDA(cudaEventCreate(&e1));
-    }
+    if (stats) CPT_NEED(need_host(s->ctx));
+    const cudaEvent_t* ev = s->ctx->time;   // lbvh_build's five, then one after the layout
     uint32_t ne = s->n_lights + s->n_spheres;
     cpt_status st = lbvh_build(ne, s->extra_c, s->extra_box, s->n_tris, s->tri_f32, s->tri_f64, s->bmin, s->bmax,
-                               buffers_of(s), s->scratch, s->scratch_bytes, stream, stats ? &tm : nullptr);
+                               buffers_of(s), s->scratch, s->scratch_bytes, stream, stats ? ev : nullptr);
     if (st != CPT_OK) return st;
-    if (stats) CPT_CUDA(cudaEventRecord(e0, stream));
     uint32_t num_wide = 0;
     st = make_layout(s, stream, &num_wide);
     if (st != CPT_OK) return st;
     s->built = true;
     if (stats) {
-        CPT_CUDA(cudaEventRecord(e1, stream));
-        CPT_CUDA(cudaEventSynchronize(e1));
         std::memset(stats, 0, sizeof *stats);
+        if (s->n == 0) return CPT_OK;
+        CPT_CUDA(cudaEventRecord(ev[5], stream));
+        CPT_CUDA(cudaEventSynchronize(ev[5]));
         stats->num_prims = s->n;
         stats->num_wide_nodes = num_wide;
-        stats->ms_prep = tm.ms_prep;
-        stats->ms_sort = tm.ms_sort;
-        stats->ms_emit = tm.ms_emit;
-        stats->ms_refit = tm.ms_refit;
-        CPT_CUDA(cudaEventElapsedTime(&stats->ms_collapse, e0, e1));
-        stats->ms_total = tm.ms_prep + tm.ms_sort + tm.ms_emit + tm.ms_refit + stats->ms_collapse;
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
+        CPT_CUDA(cudaEventElapsedTime(&stats->ms_prep, ev[0], ev[1]));
+        CPT_CUDA(cudaEventElapsedTime(&stats->ms_sort, ev[1], ev[2]));
+        CPT_CUDA(cudaEventElapsedTime(&stats->ms_emit, ev[2], ev[3]));
+        CPT_CUDA(cudaEventElapsedTime(&stats->ms_refit, ev[3], ev[4]));
+        CPT_CUDA(cudaEventElapsedTime(&stats->ms_collapse, ev[4], ev[5]));
+        stats->ms_total = stats->ms_prep + stats->ms_sort + stats->ms_emit + stats->ms_refit + stats->ms_collapse;
     }
     return CPT_OK;
 }
@@ -741,12 +817,9 @@ CPT_EXPORT cpt_status cpt_lbvh_refit(cpt_scene* s, void* stream_, cpt_bvh_stats*
     if (!s) return fail(CPT_ERR_INVALID_ARGUMENT, "cpt_lbvh_refit: scene is NULL");
     if (!s->built) return fail(CPT_ERR_NOT_BUILT, "cpt_lbvh_refit: build the LBVH first");
     cudaStream_t stream = (cudaStream_t)stream_;
-    cudaEvent_t e0, e1;
-    if (stats) {
-        CPT_CUDA(cudaEventCreate(&e0));
-        CPT_CUDA(cudaEventCreate(&e1));
-        CPT_CUDA(cudaEventRecord(e0, stream));
-    }
+    if (stats) CPT_NEED(need_host(s->ctx));
+    const cudaEvent_t e0 = s->ctx->time[0], e1 = s->ctx->time[1];
+    if (stats) CPT_CUDA(cudaEventRecord(e0, stream));
     uint32_t ne = s->n_lights + s->n_spheres;
     cpt_status st = lbvh_leaf_boxes(ne, s->extra_box, s->n_tris, s->tri_f32, s->tri_f64, s->order, s->leaf_box, s->n, stream);
     if (st != CPT_OK) return st;
@@ -761,8 +834,6 @@ CPT_EXPORT cpt_status cpt_lbvh_refit(cpt_scene* s, void* stream_, cpt_bvh_stats*
         stats->num_prims = s->n;
         CPT_CUDA(cudaEventElapsedTime(&stats->ms_refit, e0, e1));
         stats->ms_total = stats->ms_refit;
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
     }
     return CPT_OK;
 }
@@ -926,17 +997,37 @@ CPT_EXPORT cpt_status cpt_trace_closest(cpt_scene* s, const cpt_ray* rays, uint6
     cudaStream_t stream = (cudaStream_t)stream_;
     CPT_CUDA(cudaSetDevice(s->ctx->device));
     SceneView v = view_of(s);
-    if (on_device) {
-        cpt_status st = launch_trace(v, rays, n, hits, s->err, stream);
-        if (st != CPT_OK) return st;
-        return CPT_OK;
+    cpt_context* c = s->ctx;
+    if (!c->trace_resident[0]) {
+        cpt_status st = trace_grids(c->sm_count, c->trace_resident);
+        if (st != CPT_OK) {
+            c->trace_resident[0] = 0;
+            return st;
+        }
     }
+    if (on_device) return launch_trace(v, rays, n, hits, s->err, stream, c->trace_resident);
+    CPT_NEED(need_host(c));
+    if (n <= STAGED_RAYS) {
+        if (!c->staging) {
+            CPT_CUDA(cudaHostAlloc((void**)&c->staging, STAGED_RAYS * (sizeof(cpt_ray) + sizeof(cpt_hit)),
+                                   cudaHostAllocMapped));
+            CPT_CUDA(cudaHostGetDevicePointer((void**)&c->staging_dev, c->staging, 0));
+        }
+        const size_t at = STAGED_RAYS * sizeof(cpt_ray);
+        std::memcpy(c->staging, rays, n * sizeof(cpt_ray));
+        cpt_status st = launch_trace(v, (const cpt_ray*)c->staging_dev, n, (cpt_hit*)(c->staging_dev + at), s->err,
+                                     stream, c->trace_resident);
+        if (st == CPT_OK) st = check_device_error(s, stream);   // waits for the stream
+        if (st == CPT_OK) std::memcpy(hits, c->staging + at, n * sizeof(cpt_hit));
+        return st;
+    }
+    CPT_NEED(need_pool(c));
     cpt_ray* dr = nullptr;
     cpt_hit* dh = nullptr;
-    CPT_CUDA(cudaMallocAsync((void**)&dr, n * sizeof(cpt_ray), stream));
-    CPT_CUDA(cudaMallocAsync((void**)&dh, n * sizeof(cpt_hit), stream));
+    CPT_CUDA(cudaMallocFromPoolAsync((void**)&dr, n * sizeof(cpt_ray), c->pool, stream));
+    CPT_CUDA(cudaMallocFromPoolAsync((void**)&dh, n * sizeof(cpt_hit), c->pool, stream));
     CPT_CUDA(cudaMemcpyAsync(dr, rays, n * sizeof(cpt_ray), cudaMemcpyHostToDevice, stream));
-    cpt_status st = launch_trace(v, dr, n, dh, s->err, stream);
+    cpt_status st = launch_trace(v, dr, n, dh, s->err, stream, c->trace_resident);
     if (st == CPT_OK) CPT_CUDA(cudaMemcpyAsync(hits, dh, n * sizeof(cpt_hit), cudaMemcpyDeviceToHost, stream));
     cudaFreeAsync(dr, stream);
     cudaFreeAsync(dh, stream);
@@ -964,17 +1055,19 @@ CPT_EXPORT cpt_status cpt_render(cpt_scene* s, const cpt_render_params* p, const
     if (r0 < 0 || r1 > H || r0 > r1) return fail(CPT_ERR_INVALID_ARGUMENT, "cpt_render: bad row range");
     cudaStream_t stream = (cudaStream_t)stream_;
     CPT_CUDA(cudaSetDevice(s->ctx->device));
+    CPT_NEED(need_pool(s->ctx));
+    CPT_NEED(need_host(s->ctx));
     size_t np = (size_t)W * H;
     float* rgb = out->rgb;
     uint8_t* rgba8 = out->rgba8;
     float* gbuf = out->gbuffer;
     bool host = !out->on_device;
     if (host) {
-        CPT_CUDA(cudaMallocAsync((void**)&rgb, np * 12, stream));
+        CPT_CUDA(cudaMallocFromPoolAsync((void**)&rgb, np * 12, s->ctx->pool, stream));
         if (p->flags & CPT_RENDER_ACCUMULATE)
             CPT_CUDA(cudaMemcpyAsync(rgb, out->rgb, np * 12, cudaMemcpyHostToDevice, stream));
-        if (out->rgba8) CPT_CUDA(cudaMallocAsync((void**)&rgba8, np * 4, stream));
-        if (out->gbuffer) CPT_CUDA(cudaMallocAsync((void**)&gbuf, np * 32, stream));
+        if (out->rgba8) CPT_CUDA(cudaMallocFromPoolAsync((void**)&rgba8, np * 4, s->ctx->pool, stream));
+        if (out->gbuffer) CPT_CUDA(cudaMallocFromPoolAsync((void**)&gbuf, np * 32, s->ctx->pool, stream));
     }
     RenderArgs a;
     a.spp = p->spp;
@@ -992,11 +1085,7 @@ CPT_EXPORT cpt_status cpt_render(cpt_scene* s, const cpt_render_params* p, const
     a.ray_counter = s->ray_counter;
     a.err = s->err;
     a.iter_limit = s->ctx->iter_limit;
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
-    if (stats) {
-        CPT_CUDA(cudaEventCreate(&e0));
-        CPT_CUDA(cudaEventCreate(&e1));
-    }
+    const cudaEvent_t e0 = s->ctx->time[0], e1 = s->ctx->time[1];
     CPT_CUDA(cudaMemsetAsync(s->ray_counter, 0, sizeof(unsigned long long), stream));
     if (stats) CPT_CUDA(cudaEventRecord(e0, stream));
     cpt_status st = CPT_OK;
@@ -1025,19 +1114,17 @@ CPT_EXPORT cpt_status cpt_render(cpt_scene* s, const cpt_render_params* p, const
     }
     if (st != CPT_OK) return st;
     if (stats) {
-        unsigned long long rays = 0;
-        CPT_CUDA(cudaMemcpyAsync(&rays, s->ray_counter, sizeof rays, cudaMemcpyDeviceToHost, stream));
-        CPT_CUDA(cudaEventSynchronize(e1));
+        CPT_CUDA(cudaMemcpyAsync(&s->ctx->host->rays, s->ray_counter, sizeof s->ctx->host->rays, cudaMemcpyDeviceToHost,
+                                 stream));
+        st = check_device_error(s, stream);   // waits for the stream
         float ms = 0;
         CPT_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        CPT_CUDA(cudaStreamSynchronize(stream));
-        stats->rays = rays;
+        stats->rays = s->ctx->host->rays;
         stats->paths = (uint64_t)(r1 - r0) * W * p->spp;
         stats->ms = ms;
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
+        return st;
     }
-    if (host || stats) return check_device_error(s, stream);
+    if (host) return check_device_error(s, stream);
     return CPT_OK;
 }
 
@@ -1072,6 +1159,8 @@ CPT_EXPORT cpt_status cpt_render_batch(cpt_context* ctx, const cpt_render_job* j
     }
     cudaStream_t stream = (cudaStream_t)stream_;
     CPT_CUDA(cudaSetDevice(ctx->device));
+    CPT_NEED(need_pool(ctx));
+    CPT_NEED(need_host(ctx));
     std::vector<SceneView> views(count);
     std::vector<RenderArgs> args(count);
     std::vector<void*> temps;
@@ -1103,7 +1192,7 @@ CPT_EXPORT cpt_status cpt_render_batch(cpt_context* ctx, const cpt_render_job* j
         if (!j.output.on_device) {   // device copies of host outputs for the duration of the call
             auto tmp = [&](auto** dst, size_t bytes, const void* init) {
                 void* d = nullptr;
-                cudaError_t e = cudaMallocAsync(&d, bytes, stream);
+                cudaError_t e = cudaMallocFromPoolAsync(&d, bytes, ctx->pool, stream);
                 if (e == cudaSuccess && init) e = cudaMemcpyAsync(d, init, bytes, cudaMemcpyHostToDevice, stream);
                 if (e != cudaSuccess) {
                     if (d) cudaFreeAsync(d, stream);
@@ -1134,11 +1223,7 @@ CPT_EXPORT cpt_status cpt_render_batch(cpt_context* ctx, const cpt_render_job* j
             return st;
         }
     }
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
-    if (stats) {
-        CPT_CUDA(cudaEventCreate(&e0));
-        CPT_CUDA(cudaEventCreate(&e1));
-    }
+    const cudaEvent_t e0 = ctx->time[0], e1 = ctx->time[1];
     CPT_CUDA(cudaMemsetAsync(s0->ray_counter, 0, sizeof(unsigned long long), stream));
     if (stats) CPT_CUDA(cudaEventRecord(e0, stream));
     st = launch_render_wavefront_batch(views.data(), args.data(), (int)count, stream, ctx->wf);
@@ -1160,17 +1245,15 @@ CPT_EXPORT cpt_status cpt_render_batch(cpt_context* ctx, const cpt_render_job* j
     release();
     if (st != CPT_OK) return st;
     if (stats) {
-        unsigned long long rays = 0;
-        CPT_CUDA(cudaMemcpyAsync(&rays, s0->ray_counter, sizeof rays, cudaMemcpyDeviceToHost, stream));
-        CPT_CUDA(cudaEventSynchronize(e1));
+        CPT_CUDA(cudaMemcpyAsync(&ctx->host->rays, s0->ray_counter, sizeof ctx->host->rays, cudaMemcpyDeviceToHost,
+                                 stream));
+        st = check_device_error(s0, stream);   // waits for the stream
         float ms = 0;
         CPT_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        CPT_CUDA(cudaStreamSynchronize(stream));
-        stats->rays = rays;
+        stats->rays = ctx->host->rays;
         stats->paths = paths;
         stats->ms = ms;
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
+        return st;
     }
     return check_device_error(s0, stream);
 }

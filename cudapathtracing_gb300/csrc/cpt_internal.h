@@ -39,18 +39,15 @@ struct LbvhBuffers {
     float4* leaf_box;     // 2*N, sorted leaf order
 };
 
-struct LbvhTimings {
-    float ms_prep, ms_sort, ms_emit, ms_refit;
-};
-
 size_t lbvh_scratch_bytes(uint32_t n);
 
 // Builds keys/order/topology/boxes.  Primitive i < n_extra takes its centroid (double) and
-// box from the extra arrays; primitive n_extra + t is triangle t of tri_f32 or tri_f64.
+// box from the extra arrays; primitive n_extra + t is triangle t of tri_f32 or tri_f64.  stages
+// (optional): five events recorded before prep and after prep, sort, emission and refit.
 cpt_status lbvh_build(uint32_t n_extra, const double* extra_centroid, const float4* extra_box, uint32_t n_tri,
                       const float* tri_f32, const double* tri_f64, const double smin[3], const double smax[3],
                       const LbvhBuffers& out, void* scratch, size_t scratch_bytes, cudaStream_t stream,
-                      LbvhTimings* timings);
+                      const cudaEvent_t* stages);
 
 // Range-union refit only (topology and ranges kept, boxes recomputed from new leaf boxes).
 cpt_status lbvh_refit(uint32_t n, const LbvhBuffers& out, void* scratch, size_t scratch_bytes, cudaStream_t stream);
@@ -69,8 +66,10 @@ cpt_status build_trace_layout(uint32_t n, uint32_t n_lights, uint32_t n_spheres,
                               float4* leaf_rec, cudaStream_t stream, bool compressed = false);
 
 // ---- trace / render launchers (trace.cu, render.cu)
+// resident: blocks of the trace kernels (binary, 8-wide) that fit the device at once.
 cpt_status launch_trace(const SceneView& view, const cpt_ray* rays, uint64_t n, cpt_hit* hits, int* d_err,
-                        cudaStream_t stream);
+                        cudaStream_t stream, const int resident[2]);
+cpt_status trace_grids(int sm_count, int resident[2]);
 
 struct RenderArgs {
     int spp, estimator, max_depth, rr_depth;
@@ -106,8 +105,10 @@ struct WavefrontTuning {
     bool material_sort;          // shade slots binned by the material their ray hit
     int max_replays;             // iteration chunks replayed before the render gives up (CPT_ERR_TIMEOUT)
     cudaStream_t capture_stream; // non-default stream used only to capture the iteration graph
-    cudaStream_t side_stream;    // second capture stream: shadow rays traced beside extension rays
-    cudaEvent_t fork, join;      // capture-time dependencies between the two streams
+    cudaStream_t side_stream;    // second stream: shadow rays traced beside extension rays
+    cudaEvent_t fork, join;      // dependencies between the two streams
+    cudaMemPool_t pool;          // the context's workspace pool
+    int* host_cnt;               // pinned: the counters read back between chunks of iterations
 };
 
 cpt_status launch_render_wavefront(const SceneView& view, const RenderArgs& args, cudaStream_t stream,
@@ -120,7 +121,7 @@ cpt_status launch_render_wavefront_batch(const SceneView* views, const RenderArg
 // The reference's joint-bilateral and temporal filters (filter.cu); device buffers.
 DevCamera camera_of(const cpt_camera& c);
 cpt_status filter_bilateral(const float* rgb, const float* gbuf, float* out, int W, int H, const cpt_filter_params& p,
-                            cudaStream_t stream);
+                            cudaStream_t stream, cudaMemPool_t pool);
 cpt_status filter_temporal(float* rgb, const float* prev, const float* gbuf, const cpt_camera& cam,
                            const cpt_camera& prev_cam, float alpha, cudaStream_t stream);
 

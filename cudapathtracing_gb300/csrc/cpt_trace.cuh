@@ -548,7 +548,9 @@ __device__ __forceinline__ uint32_t lane_mask_lt()
 // traced by the lane.
 constexpr int CPT_REFILL = 8;
 
-template <typename Walk, typename Views, typename Load, typename Store>
+// SPREAD: fewer items than lanes are spread over all warps (a warp with one ray steps without
+// divergence, so a few rays are answered in the time of their own steps).
+template <typename Walk, bool SPREAD = false, typename Views, typename Load, typename Store>
 __device__ __forceinline__ uint32_t trace_items_walk(const Views& views, int n, int* fetch, int* err, Load load,
                                                      Store store)
 {
@@ -558,12 +560,17 @@ __device__ __forceinline__ uint32_t trace_items_walk(const Views& views, int n, 
     int item = -1, scene = 0;
     bool exhausted = false;
     uint32_t rays = 0;
+    int lanes = 32;   // of this warp that take items
+    if (SPREAD) {
+        const int warps = (int)(gridDim.x * (blockDim.x >> 5));
+        lanes = min(32, (n + warps - 1) / warps);
+    }
     for (;;) {
-        const bool idle = item < 0;
+        const bool idle = item < 0 && (!SPREAD || lane < lanes);
         const uint32_t m = __ballot_sync(0xffffffffu, idle);
         // refill once at least CPT_REFILL lanes are idle (one atomic and one divergent ray load per
         // batch instead of per finished ray): 1 -> 8 lanes is +10 % on the 1080p render (16: same)
-        if (__popc(m) >= CPT_REFILL && !exhausted) {
+        if (__popc(m) >= (SPREAD ? min(CPT_REFILL, lanes) : CPT_REFILL) && !exhausted) {
             int base = 0;
             if (lane == 0) base = atomicAdd(fetch, __popc(m));
             base = __shfl_sync(0xffffffffu, base, 0);
@@ -590,30 +597,19 @@ __device__ __forceinline__ uint32_t trace_items_walk(const Views& views, int n, 
     return rays;
 }
 
-template <bool ANY, typename Stack, typename Views, typename Load, typename Store>
+template <bool ANY, typename Stack, bool SPREAD = false, typename Views, typename Load, typename Store>
 __device__ __forceinline__ uint32_t trace_items_bvh2_views(const Views& views, int n, int* fetch, int* err, Load load,
                                                            Store store)
 {
-    return trace_items_walk<Bvh2Walk<ANY ? Q_ANY : Q_CLOSEST, Stack>>(views, n, fetch, err, load, store);
+    return trace_items_walk<Bvh2Walk<ANY ? Q_ANY : Q_CLOSEST, Stack>, SPREAD>(views, n, fetch, err, load, store);
 }
 
 // Dynamic fetching over the 8-wide BVH (the same refill policy).
-template <bool ANY, typename Stack64, typename Views, typename Load, typename Store>
+template <bool ANY, typename Stack64, bool SPREAD = false, typename Views, typename Load, typename Store>
 __device__ __forceinline__ uint32_t trace_items_wide_views(const Views& views, int n, int* fetch, int* err, Load load,
                                                            Store store)
 {
-    return trace_items_walk<WideWalk<ANY ? Q_ANY : Q_CLOSEST, Stack64>>(views, n, fetch, err, load, store);
-}
-
-// The same over one scene.
-template <bool ANY, typename Stack = ShortStack, typename Load, typename Store>
-__device__ __forceinline__ uint32_t trace_items_bvh2(const SceneView& s, int n, int* fetch, int* err, Load load,
-                                                     Store store)
-{
-    return trace_items_bvh2_views<ANY, Stack>(
-        [&](int) -> const SceneView& { return s; }, n, fetch, err,
-        [&](int i, float3& o, float3& d, float& tmn, float& tmx, int& skip, int&) { load(i, o, d, tmn, tmx, skip); },
-        [&](int i, const Hit& h, int) { store(i, h); });
+    return trace_items_walk<WideWalk<ANY ? Q_ANY : Q_CLOSEST, Stack64>, SPREAD>(views, n, fetch, err, load, store);
 }
 
 // Closest hit over [tmin (boxes), tmax]; false on a miss.  WIDE selects the traversal layout at

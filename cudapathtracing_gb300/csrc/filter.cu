@@ -122,7 +122,7 @@ inline int image_height(const cpt_camera& c)
 }  // namespace
 
 cpt_status filter_bilateral(const float* rgb, const float* gbuf, float* out, int W, int H, const cpt_filter_params& p,
-                            cudaStream_t stream)
+                            cudaStream_t stream, cudaMemPool_t pool)
 {
     if (W <= 0 || H <= 0) return CPT_OK;
     if (p.radius < 0 || p.radius > 256 || !(p.sigma_g > 0) || !(p.sigma_r > 0) || !(p.sigma_n > 0) || !(p.sigma_d > 0))
@@ -136,7 +136,7 @@ cpt_status filter_bilateral(const float* rgb, const float* gbuf, float* out, int
     k.kd = 1.0f / (2.0f * p.sigma_d * p.sigma_d);
     k.radius = p.radius;
     float* tmp = nullptr;
-    CPT_CUDA(cudaMallocAsync((void**)&tmp, (size_t)W * H * 3 * sizeof(float), stream));
+    CPT_CUDA(cudaMallocFromPoolAsync((void**)&tmp, (size_t)W * H * 3 * sizeof(float), pool, stream));
     dim3 block(32, 8), grid((W + 31) / 32, (H + 7) / 8);
     k_bilateral_pass<true><<<grid, block, 0, stream>>>(rgb, (const float4*)gbuf, tmp, W, H, k);
     k_bilateral_pass<false><<<grid, block, 0, stream>>>(tmp, (const float4*)gbuf, out, W, H, k);

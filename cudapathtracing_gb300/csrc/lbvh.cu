@@ -958,7 +958,7 @@ size_t lbvh_scratch_bytes(uint32_t n) { return layout_for(std::max(n, 1u)).total
 cpt_status lbvh_build(uint32_t n_extra, const double* extra_centroid, const float4* extra_box, uint32_t n_tri,
                       const float* tri_f32, const double* tri_f64, const double smin_in[3], const double smax_in[3],
                       const LbvhBuffers& out, void* scratch, size_t scratch_bytes, cudaStream_t stream,
-                      LbvhTimings* timings)
+                      const cudaEvent_t* stages)
 {
     uint64_t n64 = (uint64_t)n_extra + n_tri;
     if (n64 == 0) return CPT_OK;
@@ -995,10 +995,7 @@ cpt_status lbvh_build(uint32_t n_extra, const double* extra_centroid, const floa
         smax = make_double3(20.0, 20.0, 20.0);
     }
 
-    cudaEvent_t ev[5];
-    if (timings)
-        for (auto& e : ev) CPT_CUDA(cudaEventCreate(&e));
-    if (timings) CPT_CUDA(cudaEventRecord(ev[0], stream));
+    if (stages) CPT_CUDA(cudaEventRecord(stages[0], stream));
     auto axis = [](double mn, double mx) {
         MortonAxis m;
         m.mn = mn;
@@ -1019,7 +1016,7 @@ cpt_status lbvh_build(uint32_t n_extra, const double* extra_centroid, const floa
                                                               ay, az, kin, vin, box_unsorted);
     CPT_CUDA(cudaGetLastError());
     add_launches(1);
-    if (timings) CPT_CUDA(cudaEventRecord(ev[1], stream));
+    if (stages) CPT_CUDA(cudaEventRecord(stages[1], stream));
 
     // Radix sort: RS_PASSES passes of RS_BITS bits, ending in code0/val0 (= out.order).
     CPT_CUDA(cudaMemsetAsync(totals, 0, RS_PASSES * RS_BINS * 4, stream));
@@ -1040,7 +1037,7 @@ cpt_status lbvh_build(uint32_t n_extra, const double* extra_centroid, const floa
     }
     CPT_CUDA(cudaGetLastError());
     add_launches(1 + 3 * RS_PASSES);
-    if (timings) CPT_CUDA(cudaEventRecord(ev[2], stream));
+    if (stages) CPT_CUDA(cudaEventRecord(stages[2], stream));
 
     // Emission + sorted leaf boxes.
     if (n > 1) k_emit<<<blocks_for(n - 1, 256), 256, 0, stream>>>(kin, vin, (int)n, out.child, out.range);
@@ -1050,19 +1047,11 @@ cpt_status lbvh_build(uint32_t n_extra, const double* extra_centroid, const floa
                                                                     out.keys, levels, depth);
     CPT_CUDA(cudaGetLastError());
     add_launches((n > 1 ? 1 : 0) + 1);
-    if (timings) CPT_CUDA(cudaEventRecord(ev[3], stream));
+    if (stages) CPT_CUDA(cudaEventRecord(stages[3], stream));
 
     cpt_status st = refit_from_leaves(n, SL, base, out.range, out.node_box, out.leaf_box, stream, depth);
     if (st != CPT_OK) return st;
-    if (timings) {
-        CPT_CUDA(cudaEventRecord(ev[4], stream));
-        CPT_CUDA(cudaEventSynchronize(ev[4]));
-        CPT_CUDA(cudaEventElapsedTime(&timings->ms_prep, ev[0], ev[1]));
-        CPT_CUDA(cudaEventElapsedTime(&timings->ms_sort, ev[1], ev[2]));
-        CPT_CUDA(cudaEventElapsedTime(&timings->ms_emit, ev[2], ev[3]));
-        CPT_CUDA(cudaEventElapsedTime(&timings->ms_refit, ev[3], ev[4]));
-        for (auto& e : ev) cudaEventDestroy(e);
-    }
+    if (stages) CPT_CUDA(cudaEventRecord(stages[4], stream));
     return CPT_OK;
 }
 

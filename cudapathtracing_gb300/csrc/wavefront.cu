@@ -1030,7 +1030,7 @@ cpt_status run_wavefront(const SceneView& view, const RenderArgs& args, const st
     w.n_jobs = MULTI ? (int)J.size() : 0;
     size_t bytes = wf_bytes(M, L, n_parts, n_gs, tune.material_sort, w.n_jobs);
     char* base = nullptr;
-    CPT_CUDA(cudaMallocAsync((void**)&base, bytes, stream));
+    CPT_CUDA(cudaMallocFromPoolAsync((void**)&base, bytes, tune.pool, stream));
     char* p = base;
     size_t left = bytes;
     size_t ml = (size_t)M * L;
@@ -1087,7 +1087,7 @@ cpt_status run_wavefront(const SceneView& view, const RenderArgs& args, const st
             return cuda_fail(ce, "cudaGraphInstantiate");
         }
     }
-    int host_cnt[7];
+    int* const host_cnt = tune.host_cnt;
     const int max_chunks = tune.max_replays;
     bool drained = false;
     int chunk = 0;
@@ -1097,10 +1097,9 @@ cpt_status run_wavefront(const SceneView& view, const RenderArgs& args, const st
         const int grid = std::min((M + PATHS_THREADS - 1) / PATHS_THREADS, tune.grid_paths);
         k<<<grid, PATHS_THREADS, smem, stream>>>(view, w, args, 0, CHUNK * chunk, CHUNK * max_chunks);
         add_launches(1);
-        int left = 0;
-        CPT_CUDA(cudaMemcpyAsync(&left, w.cnt + CNT_LEFT, sizeof left, cudaMemcpyDeviceToHost, stream));
+        CPT_CUDA(cudaMemcpyAsync(host_cnt, w.cnt + CNT_LEFT, sizeof(int), cudaMemcpyDeviceToHost, stream));
         CPT_CUDA(cudaStreamSynchronize(stream));
-        drained = left == 0;
+        drained = host_cnt[0] == 0;
         return CPT_OK;
     };
     if (paths_only) {
@@ -1113,7 +1112,7 @@ cpt_status run_wavefront(const SceneView& view, const RenderArgs& args, const st
             enqueue_chunk<MULTI>(view, w, args, gt, bt, gs, bs, tune.short_stack, stream, nullptr);
         }
         add_launches(4 * CHUNK);
-        CPT_CUDA(cudaMemcpyAsync(host_cnt, w.cnt, sizeof host_cnt, cudaMemcpyDeviceToHost, stream));
+        CPT_CUDA(cudaMemcpyAsync(host_cnt, w.cnt, 7 * sizeof(int), cudaMemcpyDeviceToHost, stream));
         CPT_CUDA(cudaStreamSynchronize(stream));
         if (host_cnt[0] == 0 && host_cnt[2] == 0 && host_cnt[4] == 0) {
             drained = true;
