@@ -453,10 +453,17 @@ SceneView view_of(const cpt_scene* s)
     return v;
 }
 
+// Binary traversal nodes (either format), allocated on first use.
+cpt_status need_nodes(cpt_scene* s)
+{
+    return s->nodes || s->n < 2 ? CPT_OK : dalloc(&s->nodes, 4 * (size_t)(s->n - 1));
+}
+
 // Traversal layout for the context's BVH width: the compressed 8-wide BVH (collapse in wide.cu,
 // using the LBVH scratch for its task queues) or the BVH2 node array; leaf records in the
 // matching order.  Buffers are allocated on first use.
-cpt_status make_layout(cpt_scene* s, cudaStream_t stream, uint32_t* num_wide)
+// `nodes_ready`: the build has written the 64-byte binary nodes along with the hierarchy.
+cpt_status make_layout(cpt_scene* s, cudaStream_t stream, uint32_t* num_wide, bool nodes_ready)
 {
     uint32_t n = s->n;
     uint32_t ni = n > 1 ? n - 1 : 0;
@@ -475,15 +482,13 @@ cpt_status make_layout(cpt_scene* s, cudaStream_t stream, uint32_t* num_wide)
         return build_trace_layout(n, s->n_lights, s->n_spheres, s->child, s->node_box, s->leaf_box, wide_order,
                                   s->tri_f32, s->tri_f64, s->spheres, nullptr, s->leaf_rec, stream);
     }
-    if (!s->nodes && ni) {
-        cpt_status st = dalloc(&s->nodes, 4 * (size_t)ni);
-        if (st != CPT_OK) return st;
-    }
+    cpt_status st = need_nodes(s);
+    if (st != CPT_OK) return st;
     s->width = 2;
     s->node_q = s->ctx->bvh2_compressed;
     if (num_wide) *num_wide = 0;
     return build_trace_layout(n, s->n_lights, s->n_spheres, s->child, s->node_box, s->leaf_box, s->order, s->tri_f32,
-                              s->tri_f64, s->spheres, s->nodes, s->leaf_rec, stream, s->node_q);
+                              s->tri_f64, s->spheres, nodes_ready ? nullptr : s->nodes, s->leaf_rec, stream, s->node_q);
 }
 
 LbvhBuffers buffers_of(cpt_scene* s)
@@ -495,6 +500,7 @@ LbvhBuffers buffers_of(cpt_scene* s)
     b.range = s->range;
     b.node_box = s->node_box;
     b.leaf_box = s->leaf_box;
+    b.nodes = nullptr;
     return b;
 }
 
@@ -788,11 +794,17 @@ CPT_EXPORT cpt_status cpt_lbvh_build(cpt_scene* s, void* stream_, cpt_bvh_stats*
     if (stats) CPT_NEED(need_host(s->ctx));
     const cudaEvent_t* ev = s->ctx->time;   // lbvh_build's five, then one after the layout
     uint32_t ne = s->n_lights + s->n_spheres;
-    cpt_status st = lbvh_build(ne, s->extra_c, s->extra_box, s->n_tris, s->tri_f32, s->tri_f64, s->bmin, s->bmax,
-                               buffers_of(s), s->scratch, s->scratch_bytes, stream, stats ? ev : nullptr);
+    LbvhBuffers out = buffers_of(s);
+    if (s->n > 1 && s->ctx->bvh_width == 2 && !s->ctx->bvh2_compressed) {
+        cpt_status st = need_nodes(s);
+        if (st != CPT_OK) return st;
+        out.nodes = s->nodes;
+    }
+    cpt_status st = lbvh_build(ne, s->extra_c, s->extra_box, s->n_tris, s->tri_f32, s->tri_f64, s->bmin, s->bmax, out,
+                               s->scratch, s->scratch_bytes, stream, stats ? ev : nullptr);
     if (st != CPT_OK) return st;
     uint32_t num_wide = 0;
-    st = make_layout(s, stream, &num_wide);
+    st = make_layout(s, stream, &num_wide, out.nodes != nullptr);
     if (st != CPT_OK) return st;
     s->built = true;
     if (stats) {
@@ -825,7 +837,7 @@ CPT_EXPORT cpt_status cpt_lbvh_refit(cpt_scene* s, void* stream_, cpt_bvh_stats*
     if (st != CPT_OK) return st;
     st = lbvh_refit(s->n, buffers_of(s), s->scratch, s->scratch_bytes, stream);
     if (st != CPT_OK) return st;
-    st = make_layout(s, stream, nullptr);
+    st = make_layout(s, stream, nullptr, false);
     if (st != CPT_OK) return st;
     if (stats) {
         CPT_CUDA(cudaEventRecord(e1, stream));

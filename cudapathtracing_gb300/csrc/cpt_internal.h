@@ -37,6 +37,7 @@ struct LbvhBuffers {
     int2* range;          // N-1: (first, last), optional
     float4* node_box;     // 2*(N-1): min (w = 0), max
     float4* leaf_box;     // 2*N, sorted leaf order
+    float4* nodes;        // 4*(N-1), optional: the 64-byte traversal nodes, written with the hierarchy
 };
 
 size_t lbvh_scratch_bytes(uint32_t n);

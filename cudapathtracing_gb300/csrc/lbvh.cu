@@ -3,17 +3,20 @@
 //   k_prep        centroid (FP64) + Morton code + leaf box per primitive
 //                 (generateMortonCodes Device.cuh:134-142, morton3D BVH.cuh:23-41,
 //                  Hittable ctors Hittable.cuh:456-462)
-//   radix sort    stable LSD over the 30-bit codes, three 10-bit digits, per-tile ranking with
-//                 __match_any_sync (replaces thrust::sort_by_key Device.cuh:187-189: keys are
+//   radix sort    stable LSD over the 30-bit codes, four 8-bit digits, one launch per digit: tiles
+//                 take their offsets from the tiles before them while those are still running
+//                 (chained scan; replaces thrust::sort_by_key Device.cuh:187-189: keys are
 //                 code<<32|index, so a stable sort of codes with ascending indices is the
 //                 same permutation)
-//   k_emit        Karras 2012 range/split per internal node (generateHierarchy BVH.cuh:174-241)
-//   refit         atomic-free: an internal node covers the contiguous sorted leaves
-//                 [first, last], so its box is a range union, answered from a 4-ary pyramid
-//                 of unions of the leaf boxes (replaces the serial constructAABB BVH.cuh:243-280;
-//                 min/max is exact, so the boxes equal the pairwise unions)
+//   k_tree        the Karras 2012 hierarchy with its boxes, a thread per node
+//                 (generateHierarchy BVH.cuh:174-241, constructAABB BVH.cuh:243-280)
+//   refit         (moved vertices, same topology) atomic-free: an internal node covers the
+//                 contiguous sorted leaves [first, last], so its box is a range union, answered
+//                 from a 4-ary pyramid of unions of the leaf boxes (min/max is exact, so the boxes
+//                 equal the pairwise unions)
 //
 // All boxes are FP32 rounded outwards from the reference's FP64 boxes.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -22,20 +25,17 @@
 #include "cpt_internal.h"
 #include "cpt_quant.cuh"
 
+namespace cg = cooperative_groups;
+
 namespace cpt {
 
 namespace {
 
-constexpr int RS_THREADS = 256;
-constexpr int RS_WARPS = RS_THREADS / 32;
-constexpr int RS_ITEMS = 16;
-constexpr int RS_TILE = RS_THREADS * RS_ITEMS;   // 4096 keys per tile
-constexpr int RS_BITS = 10;
-constexpr int RS_BINS = 1 << RS_BITS;            // 1024 digits
+constexpr int RS_BITS = 8;
+constexpr int RS_BINS = 1 << RS_BITS;
 constexpr uint32_t RS_MASK = RS_BINS - 1;
-constexpr int RS_PASSES = 3;                     // bits 0-9, 10-19, 20-29: the whole 30-bit code
-constexpr int RS_DPT = RS_BINS / RS_THREADS;     // digits per thread in the per-tile scans
-static_assert(RS_BITS * RS_PASSES >= 30 && RS_BINS % RS_THREADS == 0, "radix digits");
+constexpr int RS_PASSES = 4;                     // bits 0-7, 8-15, 16-23, 24-31: the whole 30-bit code
+static_assert(RS_BITS * RS_PASSES >= 30 && RS_PASSES % 2 == 0, "radix digits");
 
 __device__ __forceinline__ uint32_t expand_bits(uint32_t v)   // BVH.cuh:12-19
 {
@@ -291,14 +291,21 @@ __device__ __forceinline__ void tri_box(const float p[9], float4& bmin, float4& 
     bmax = make_float4(pad_fp32<true>(mx[0]), pad_fp32<true>(mx[1]), pad_fp32<true>(mx[2]), 0.f);
 }
 
+// Codes and boxes of all primitives, and (they do not depend on the order) the digit totals of every
+// sort pass: totals[pass][digit].
+constexpr int PREP_THREADS = 256;
+constexpr unsigned PREP_BLOCKS = 152 * 8;   // each adds its 1,024 digit counts once
 template <typename VT>
-__global__ void k_prep(uint32_t n_extra, const double* __restrict__ extra_c, const float4* __restrict__ extra_box,
+__global__ void __launch_bounds__(PREP_THREADS) k_prep(uint32_t n_extra, const double* __restrict__ extra_c, const float4* __restrict__ extra_box,
                        uint32_t n_tri, const VT* __restrict__ tri_v, MortonAxis ax, MortonAxis ay, MortonAxis az,
-                       uint32_t* __restrict__ code, uint32_t* __restrict__ idx, float4* __restrict__ box)
+                       uint32_t* __restrict__ code, float4* __restrict__ box, uint32_t* __restrict__ totals)
 {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t n = n_extra + n_tri;
-    if (i >= n) return;
+    __shared__ uint32_t hist[RS_PASSES][RS_BINS];
+    for (int t = threadIdx.x; t < RS_PASSES * RS_BINS; t += PREP_THREADS) (&hist[0][0])[t] = 0;
+    __syncthreads();
+    const uint32_t n = n_extra + n_tri;
+    for (uint64_t i64 = blockIdx.x * (uint64_t)PREP_THREADS + threadIdx.x; i64 < n; i64 += gridDim.x * (uint64_t)PREP_THREADS) {
+    const uint32_t i = (uint32_t)i64;
     float4 bmin, bmax;
     uint32_t xx, yy, zz;
     if (i < n_extra) {
@@ -324,10 +331,18 @@ __global__ void k_prep(uint32_t n_extra, const double* __restrict__ extra_c, con
         yy = morton_axis(c[1], ay.mn, ay.mx);
         zz = morton_axis(c[2], az.mn, az.mx);
     }
-    code[i] = expand_bits(xx) * 4 + expand_bits(yy) * 2 + expand_bits(zz);
-    idx[i] = i;
+    const uint32_t c = expand_bits(xx) * 4 + expand_bits(yy) * 2 + expand_bits(zz);
+    code[i] = c;
     box[2ull * i] = bmin;
     box[2ull * i + 1] = bmax;
+#pragma unroll
+    for (int p = 0; p < RS_PASSES; ++p) atomicAdd(&hist[p][(c >> (RS_BITS * p)) & RS_MASK], 1u);
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < RS_PASSES * RS_BINS; t += PREP_THREADS) {
+        const uint32_t v = (&hist[0][0])[t];
+        if (v) atomicAdd(&totals[t], v);
+    }
 }
 
 template <typename VT>
@@ -358,24 +373,6 @@ __global__ void k_prim_boxes(uint32_t n_extra, const float4* __restrict__ extra_
 }
 
 // ---------------------------------------------------------------- radix sort
-// Digit totals of all passes (they do not depend on the order): totals[pass][digit].
-__global__ void k_digit_totals(const uint32_t* __restrict__ code, uint32_t n, uint32_t* __restrict__ totals)
-{
-    __shared__ uint32_t h[RS_PASSES][RS_BINS];
-    for (int t = threadIdx.x; t < RS_PASSES * RS_BINS; t += blockDim.x) (&h[0][0])[t] = 0;
-    __syncthreads();
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        uint32_t c = code[i];
-#pragma unroll
-        for (int p = 0; p < RS_PASSES; ++p) atomicAdd(&h[p][(c >> (RS_BITS * p)) & RS_MASK], 1u);
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < RS_PASSES * RS_BINS; t += blockDim.x) {
-        uint32_t v = (&h[0][0])[t];
-        if (v) atomicAdd(&totals[t], v);
-    }
-}
-
 __device__ __forceinline__ uint32_t lanemask_lt()
 {
     uint32_t m;
@@ -383,234 +380,194 @@ __device__ __forceinline__ uint32_t lanemask_lt()
     return m;
 }
 
-// Per-tile digit counts, digit-major: counts[d * num_tiles + tile].  Each warp aggregates
-// equal digits with __match_any_sync; the group leader adds to the warp's private row.
-__global__ void __launch_bounds__(RS_THREADS) k_radix_hist(const uint32_t* __restrict__ keys, uint32_t n, int shift,
-                                                           uint32_t* __restrict__ counts, uint32_t num_tiles)
+// Inclusive sum of x over the block's first RS_BINS threads (s_part: RS_BINS / 32 words; every thread
+// of the block calls it; the caller synchronises before s_part is used again).
+__device__ __forceinline__ uint32_t bins_scan(uint32_t x, uint32_t* s_part)
 {
-    __shared__ uint32_t wh[RS_WARPS][RS_BINS];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int t = threadIdx.x; t < RS_WARPS * RS_BINS; t += RS_THREADS) (&wh[0][0])[t] = 0;
-    __syncthreads();
-    const uint32_t tile = blockIdx.x;
-    const uint32_t base = tile * RS_TILE + w * 32 * RS_ITEMS;
-#pragma unroll 4
-    for (int it = 0; it < RS_ITEMS; ++it) {
-        uint32_t e = base + it * 32 + lane;
-        uint32_t d = e < n ? (keys[e] >> shift) & RS_MASK : (uint32_t)RS_BINS;
-        uint32_t peers = __match_any_sync(0xffffffffu, d);
-        if (d < (uint32_t)RS_BINS && lane == __ffs(peers) - 1) wh[w][d] += __popc(peers);
-        __syncwarp();
-    }
-    __syncthreads();
-    for (int d = threadIdx.x; d < RS_BINS; d += RS_THREADS) {
-        uint32_t s = 0;
-#pragma unroll
-        for (int k = 0; k < RS_WARPS; ++k) s += wh[k][d];
-        counts[(size_t)d * num_tiles + tile] = s;
-    }
-}
-
-// Exclusive scan of counts into global offsets.  Block d scans row d and adds the number
-// of keys with a smaller digit (from the pass's totals).
-__global__ void __launch_bounds__(256) k_radix_scan(uint32_t* __restrict__ counts, uint32_t num_tiles,
-                                                    const uint32_t* __restrict__ totals)
-{
-    __shared__ uint32_t s_part[8];
-    __shared__ uint32_t s_carry;
-    const int d = blockIdx.x;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    uint32_t b = 0;
-    for (int t = threadIdx.x; t < d; t += 256) b += totals[t];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
-    if (lane == 0) s_part[w] = b;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t s = 0;
-        for (int k = 0; k < 8; ++k) s += s_part[k];
-        s_carry = s;
-    }
-    __syncthreads();
-    uint32_t* row = counts + (size_t)d * num_tiles;
-    for (uint32_t start = 0; start < num_tiles; start += 256) {
-        uint32_t i = start + threadIdx.x;
-        uint32_t v = i < num_tiles ? row[i] : 0u;
-        uint32_t x = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        __syncthreads();
-        if (lane == 31) s_part[w] = x;
-        __syncthreads();
-        uint32_t wpre = 0;
-        for (int k = 0; k < w; ++k) wpre += s_part[k];
-        uint32_t carry = s_carry;
-        if (i < num_tiles) row[i] = carry + wpre + x - v;
-        __syncthreads();
-        if (threadIdx.x == 255) s_carry = carry + wpre + x;
-        __syncthreads();
-    }
-}
-
-// Shared memory of the scatter kernel (73,760 bytes, dynamic: three blocks per SM).
-struct ScatterSmem {
-    uint32_t wh[RS_WARPS][RS_BINS];   // per-warp digit counts, then per-warp exclusive offsets
-    uint32_t start[RS_BINS];          // tile-local start of each digit
-    uint32_t gofs[RS_BINS];           // global start of each digit's run of this tile
-    uint32_t keys[RS_TILE];
-    uint32_t vals[RS_TILE];
-    uint32_t wsum[RS_WARPS];
-};
-
-// Stable scatter: rank each key within its tile (warp-ordered, lane-ordered), stage the tile
-// in shared memory in sorted order, then write runs to their global offsets.
-__global__ void __launch_bounds__(RS_THREADS, 3) k_radix_scatter(const uint32_t* __restrict__ keys_in,
-                                                              const uint32_t* __restrict__ vals_in,
-                                                              uint32_t* __restrict__ keys_out,
-                                                              uint32_t* __restrict__ vals_out, uint32_t n, int shift,
-                                                              const uint32_t* __restrict__ offsets, uint32_t num_tiles)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    ScatterSmem& S = *reinterpret_cast<ScatterSmem*>(smem_raw);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int t = threadIdx.x; t < RS_WARPS * RS_BINS; t += RS_THREADS) (&S.wh[0][0])[t] = 0;
-    __syncthreads();
-    const uint32_t tile = blockIdx.x;
-    const uint32_t base = tile * RS_TILE + w * 32 * RS_ITEMS;
-    const uint32_t lt = lanemask_lt();
-    uint32_t k[RS_ITEMS], v[RS_ITEMS], rank[RS_ITEMS];
-#pragma unroll
-    for (int it = 0; it < RS_ITEMS; ++it) {
-        uint32_t e = base + it * 32 + lane;
-        bool valid = e < n;
-        k[it] = valid ? keys_in[e] : 0u;
-        v[it] = valid ? vals_in[e] : 0u;
-        uint32_t d = valid ? (k[it] >> shift) & RS_MASK : (uint32_t)RS_BINS;
-        uint32_t peers = __match_any_sync(0xffffffffu, d);
-        int leader = __ffs(peers) - 1;
-        uint32_t old = (lane == leader && valid) ? S.wh[w][d] : 0u;
-        old = __shfl_sync(0xffffffffu, old, leader);
-        if (lane == leader && valid) S.wh[w][d] = old + __popc(peers);
-        rank[it] = old + __popc(peers & lt);
-        __syncwarp();
-    }
-    __syncthreads();
-    // Digits RS_DPT * t .. RS_DPT * t + RS_DPT - 1 belong to thread t: exclusive prefix over warps
-    // (in place), the tile's count of each, and their exclusive prefix within the thread.
-    uint32_t local[RS_DPT];
-    uint32_t tsum = 0;
-#pragma unroll
-    for (int j = 0; j < RS_DPT; ++j) {
-        const int d = RS_DPT * threadIdx.x + j;
-        uint32_t run = 0;
-#pragma unroll
-        for (int q = 0; q < RS_WARPS; ++q) {
-            uint32_t c = S.wh[q][d];
-            S.wh[q][d] = run;
-            run += c;
-        }
-        local[j] = tsum;
-        tsum += run;
-        S.gofs[d] = offsets[(size_t)d * num_tiles + tile];
-    }
-    // Block exclusive scan of the threads' sums -> S.start.
-    uint32_t x = tsum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
         if (lane >= o) x += y;
     }
-    if (lane == 31) S.wsum[w] = x;
+    if (lane == 31 && w < RS_BINS / 32) s_part[w] = x;
     __syncthreads();
-    uint32_t wpre = 0;
-    for (int q = 0; q < w; ++q) wpre += S.wsum[q];
+    for (int q = 0; q < min(w, RS_BINS / 32); ++q) x += s_part[q];
+    return x;
+}
+
+// Progress of one (tile, digit) of a pass: nothing yet, the tile's own count, or the count over all
+// tiles up to it.  The two top bits say which, the rest is the count, so one store publishes both.
+template <typename Word>
+struct Chain {
+    static constexpr int SHIFT = sizeof(Word) * 8 - 2;
+    static constexpr Word VALUE = ((Word)1 << SHIFT) - 1;
+    static __device__ __forceinline__ Word own(uint32_t c) { return ((Word)1 << SHIFT) | c; }
+    static __device__ __forceinline__ Word total(Word c) { return ((Word)2 << SHIFT) | c; }
+};
+
+// One digit of the stable LSD sort (Adinets and Merrill, "Onesweep", 2022): a block takes the next
+// tile, ranks its keys by the digit (warp-ordered, lane-ordered), publishes its counts, adds up the
+// counts of the tiles before it (thread d for digit d) and writes its keys to their places, staged in
+// shared memory so that equal digits leave as runs.  Tiles are taken in order, so those before a tile
+// are done or running; a count that is not there after CHAIN_POLLS looks is counted from the keys
+// instead of waited for.
+//
+// The sort is bound by latency at these sizes (1.31M keys: 5 MB a buffer, in L2): one launch a digit
+// in place of three, with 8-bit digits (32-key runs, 256 counters a warp) in place of 10-bit ones.
+// 1.31M keys: 158 -> 91 us, 12,500: 91 -> 28 us.  Of the 158 us, 52 went to match instructions.  Tiles of
+// 2,048 keys took 29 us a pass (every tile adds up the hundreds running beside it) against 23.
+//
+// FIRST: the values are the positions.
+constexpr int CHAIN_POLLS = 4096;
+constexpr int CHAIN_BATCH = 8;   // tiles a thread fetches at once
+
+template <int THREADS, int ITEMS, typename Word>
+struct SortSmem {
+    uint32_t wh[THREADS / 32][RS_BINS];   // per-warp digit counts, then per-warp exclusive offsets
+    uint32_t start[RS_BINS];              // tile-local start of each digit
+    uint32_t gofs[RS_BINS];               // global start of each digit's run of this tile
+    uint32_t keys[THREADS * ITEMS], vals[THREADS * ITEMS];
+    uint32_t part0[RS_BINS / 32], part1[RS_BINS / 32];
+    uint32_t tile;
+    Word sum[THREADS / RS_BINS][RS_BINS];   // look-back: sums of the groups of threads, flagged when closed
+};
+
+template <int THREADS, int ITEMS, typename Word, bool FIRST>
+__global__ void __launch_bounds__(THREADS, 1) k_sort_digit(const uint32_t* __restrict__ keys_in,
+                                                           const uint32_t* __restrict__ vals_in,
+                                                           uint32_t* __restrict__ keys_out,
+                                                           uint32_t* __restrict__ vals_out, uint32_t n, int shift,
+                                                           const uint32_t* __restrict__ totals, Word* state,
+                                                           uint32_t* ticket)
+{
+    constexpr int TILE = THREADS * ITEMS, WARPS = THREADS / 32, GROUPS = THREADS / RS_BINS;
+    extern __shared__ __align__(16) unsigned char sort_smem[];
+    SortSmem<THREADS, ITEMS, Word>& S = *reinterpret_cast<SortSmem<THREADS, ITEMS, Word>*>(sort_smem);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, d_own = threadIdx.x;
+    const bool has_digit = d_own < RS_BINS;
+    if (threadIdx.x == 0) S.tile = atomicAdd(ticket, 1u);
+    for (int q = threadIdx.x; q < WARPS * RS_BINS; q += THREADS) (&S.wh[0][0])[q] = 0;
+    const uint32_t digit_total = has_digit ? totals[d_own] : 0u;
+    __syncthreads();
+    const uint32_t tile = S.tile;
+    const uint32_t base = tile * TILE + w * 32 * ITEMS;
+    const uint32_t lt = lanemask_lt();
+    uint32_t k[ITEMS], v[ITEMS], rank[ITEMS];
 #pragma unroll
-    for (int j = 0; j < RS_DPT; ++j) S.start[RS_DPT * threadIdx.x + j] = wpre + x - tsum + local[j];
+    for (int it = 0; it < ITEMS; ++it) {
+        const uint32_t e = base + it * 32 + lane;
+        const bool valid = e < n;
+        k[it] = valid ? keys_in[e] : 0u;
+        v[it] = FIRST ? e : (valid ? vals_in[e] : 0u);
+    }
+#pragma unroll
+    for (int it = 0; it < ITEMS; ++it) {
+        const bool valid = base + it * 32 + lane < n;
+        const uint32_t d = (k[it] >> shift) & RS_MASK;
+        // lanes with the same digit: a vote per bit (__match_any_sync takes a turn per distinct value)
+        uint32_t peers = __ballot_sync(0xffffffffu, valid);
+        if (!valid) peers = ~peers;
+#pragma unroll
+        for (int bit = 0; bit < RS_BITS; ++bit) {
+            const bool one = (d >> bit) & 1u;
+            const uint32_t votes = __ballot_sync(0xffffffffu, one);
+            peers &= one ? votes : ~votes;
+        }
+        const int leader = __ffs(peers) - 1;
+        uint32_t old = 0;
+        if (lane == leader && valid) {
+            old = S.wh[w][d];
+            S.wh[w][d] = old + __popc(peers);
+        }
+        rank[it] = __shfl_sync(0xffffffffu, old, leader) + __popc(peers & lt);
+        __syncwarp();
+    }
+    __syncthreads();
+    // thread d: exclusive prefix of digit d over the warps (in place) and its count in the tile
+    uint32_t count = 0;
+    volatile Word* mine = state + (size_t)tile * RS_BINS + d_own;
+    if (has_digit) {
+#pragma unroll 8
+        for (int q = 0; q < WARPS; ++q) {
+            const uint32_t c = S.wh[q][d_own];
+            S.wh[q][d_own] = count;
+            count += c;
+        }
+        *mine = tile ? Chain<Word>::own(count) : Chain<Word>::total(count);
+    }
+    const uint32_t tile_start = bins_scan(count, S.part0) - count;
+    const uint32_t digit_base = bins_scan(digit_total, S.part1) - digit_total;
+    Word before = 0;   // keys with this digit in earlier tiles
+    bool done = false;
+    // Windows of GROUPS x CHAIN_BATCH tiles, nearest first: group q of 256 threads adds up its
+    // CHAIN_BATCH tiles (fetched together), thread d of the first group joins the groups' sums.
+    for (uint32_t p = tile; p > 0;) {
+        const int q = threadIdx.x / RS_BINS, dg = threadIdx.x % RS_BINS;
+        Word x[CHAIN_BATCH];
+#pragma unroll
+        for (int j = 0; j < CHAIN_BATCH; ++j) {
+            const uint32_t back = q * CHAIN_BATCH + j + 1;
+            x[j] = back <= p ? *(volatile const Word*)(state + (size_t)(p - back) * RS_BINS + dg) : Chain<Word>::total(0);
+        }
+        Word sum = 0;
+        bool closed = false;
+#pragma unroll
+        for (int j = 0; j < CHAIN_BATCH; ++j) {
+            const uint32_t back = q * CHAIN_BATCH + j + 1;
+            Word y = x[j];
+            if (!closed && !(y >> Chain<Word>::SHIFT)) {
+                volatile const Word* theirs = state + (size_t)(p - back) * RS_BINS + dg;
+                for (int polls = 0; !(y >> Chain<Word>::SHIFT) && polls < CHAIN_POLLS; ++polls) y = *theirs;
+                if (!(y >> Chain<Word>::SHIFT)) {
+                    uint32_t c = 0;
+                    for (uint32_t e = (p - back) * TILE; e < (p - back + 1) * TILE; ++e)
+                        c += ((keys_in[e] >> shift) & RS_MASK) == (uint32_t)dg;
+                    y = Chain<Word>::own(c);
+                }
+            }
+            if (!closed) sum += y & Chain<Word>::VALUE;
+            closed = closed || (y >> Chain<Word>::SHIFT) == 2;
+        }
+        S.sum[q][dg] = (closed ? Chain<Word>::total(0) : Chain<Word>::own(0)) | sum;
+        __syncthreads();
+        bool open = false;
+        if (has_digit && !done) {
+#pragma unroll
+            for (int g = 0; g < GROUPS; ++g) {
+                if (done) continue;
+                before += S.sum[g][d_own] & Chain<Word>::VALUE;
+                done = (S.sum[g][d_own] >> Chain<Word>::SHIFT) == 2;
+            }
+            open = !done;
+        }
+        if (!__syncthreads_or(open)) break;
+        p -= min(p, (uint32_t)(GROUPS * CHAIN_BATCH));
+    }
+    if (has_digit) {
+        if (tile) *mine = Chain<Word>::total(before + count);
+        S.start[d_own] = tile_start;
+        S.gofs[d_own] = digit_base + (uint32_t)before;
+    }
     __syncthreads();
 #pragma unroll
-    for (int it = 0; it < RS_ITEMS; ++it) {
-        uint32_t e = base + it * 32 + lane;
-        if (e < n) {
-            uint32_t d = (k[it] >> shift) & RS_MASK;
-            uint32_t pos = S.start[d] + S.wh[w][d] + rank[it];
+    for (int it = 0; it < ITEMS; ++it) {
+        if (base + it * 32 + lane < n) {
+            const uint32_t d = (k[it] >> shift) & RS_MASK;
+            const uint32_t pos = S.start[d] + S.wh[w][d] + rank[it];
             S.keys[pos] = k[it];
             S.vals[pos] = v[it];
         }
     }
     __syncthreads();
-    uint32_t tile_n = min((uint32_t)RS_TILE, n - tile * RS_TILE);
-    for (uint32_t p = threadIdx.x; p < tile_n; p += RS_THREADS) {
-        uint32_t kk = S.keys[p];
-        uint32_t d = (kk >> shift) & RS_MASK;
-        uint32_t g = S.gofs[d] + (p - S.start[d]);
+    const uint32_t tile_n = min((uint32_t)TILE, n - tile * TILE);
+    for (uint32_t p = threadIdx.x; p < tile_n; p += THREADS) {
+        const uint32_t kk = S.keys[p];
+        const uint32_t d = (kk >> shift) & RS_MASK;
+        const uint32_t g = S.gofs[d] + (p - S.start[d]);
         keys_out[g] = kk;
         vals_out[g] = S.vals[p];
     }
-}
-
-// ---------------------------------------------------------------- Karras emission
-// The reference's keys are code << 32 | primitive (Device.cuh:187-189), so the length of the common
-// prefix of keys i and j (delta, BVH.cuh:120-128) is clz(code_i ^ code_j) when the codes differ and
-// 32 + clz(prim_i ^ prim_j) when they are equal: the primitive word is read only then.
-__device__ __forceinline__ int prefix_len(uint32_t ci, uint32_t oi, const uint32_t* __restrict__ code,
-                                          const uint32_t* __restrict__ order, int j)
-{
-    const uint32_t cj = code[j];
-    if (cj != ci) return __clz(ci ^ cj);
-    const uint32_t oj = order[j];
-    return oi == oj ? 64 : 32 + __clz(oi ^ oj);
-}
-
-__device__ __forceinline__ int delta_k(const uint32_t* code, const uint32_t* order, int n, uint32_t ci, uint32_t oi,
-                                       int j)   // BVH.cuh:120-128
-{
-    if (j < 0 || j >= n) return -1;
-    return prefix_len(ci, oi, code, order, j);
-}
-
-__global__ void k_emit(const uint32_t* __restrict__ code, const uint32_t* __restrict__ order, int n,
-                       int2* __restrict__ child, int2* __restrict__ range)
-{
-    int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= n - 1) return;
-    // determineRange (BVH.cuh:130-172)
-    const uint32_t ci = code[idx], oi = order[idx];
-    int dn = delta_k(code, order, n, ci, oi, idx + 1);
-    int dp = delta_k(code, order, n, ci, oi, idx - 1);
-    int d = (dn > dp) ? 1 : -1;
-    int dmin_ = delta_k(code, order, n, ci, oi, idx - d);
-    int lmax = 2;
-    while (delta_k(code, order, n, ci, oi, idx + lmax * d) > dmin_) lmax *= 2;
-    int l = 0;
-    for (int t = lmax / 2; t >= 1; t /= 2)
-        if (delta_k(code, order, n, ci, oi, idx + (l + t) * d) > dmin_) l += t;
-    int j = idx + l * d;
-    int first = min(idx, j), last = max(idx, j);
-    // findSplit (BVH.cuh:81-118): equal keys split in the middle, otherwise binary search for the
-    // last position that shares more than the range's common prefix with the first key
-    const uint32_t cf = code[first], of = order[first];
-    const int common = prefix_len(cf, of, code, order, last);
-    int split;
-    if (common == 64) {
-        split = (first + last) >> 1;
-    } else {
-        split = first;
-        int step = last - first;
-        do {
-            step = (step + 1) >> 1;
-            int ns = split + step;
-            if (ns < last) {
-                if (prefix_len(cf, of, code, order, ns) > common) split = ns;
-            }
-        } while (step > 1);
-    }
-    int a = (split == first) ? ~split : split;
-    int b = (split + 1 == last) ? ~(split + 1) : split + 1;
-    child[idx] = make_int2(a, b);
-    if (range) range[idx] = make_int2(first, last);
 }
 
 // ---------------------------------------------------------------- range-union refit
@@ -706,26 +663,272 @@ __global__ void __launch_bounds__(PYR_THREADS) k_pyramid(const float4* __restric
     pyramid_up(mn, mx, n, out, depth);
 }
 
-// Sorted leaf boxes, (optionally) the reference's 64-bit keys, and (when `levels` is set) the
-// first `depth` pyramid levels above them.
-__global__ void __launch_bounds__(PYR_THREADS) k_leaves(const uint32_t* __restrict__ code,
-                                                        const uint32_t* __restrict__ order, uint32_t n,
-                                                        const float4* __restrict__ box_unsorted,
-                                                        float4* __restrict__ leaf_box, uint64_t* __restrict__ keys,
-                                                        float4* __restrict__ levels, int depth)
+// ---------------------------------------------------------------- hierarchy
+// The binary LBVH and its boxes.  Between neighbouring sorted keys lies a gap, the length of their
+// common prefix; the Karras hierarchy (generateHierarchy, BVH.cuh:174-241) has one internal node per
+// gap, which splits there and covers the keys up to the nearest smaller gap on either side (all of its
+// keys share gap[split] bits, and no two of its gaps are equal).  The node a parent that splits behind
+// key s calls its left child has number s, its right child s + 1, the root 0; a node is a left child
+// when the gap behind it is longer than the one before it, so its number is `last` then and `first`
+// otherwise.
+//
+// k_tree: a block holds TREE_THREADS keys, thread t the gap behind key t.  Nearest smaller gaps come
+// from a table of minima over 2^k gaps in shared memory, boxes from a 4-ary pyramid of box unions
+// there.  Gaps whose node reaches beyond the block (about one in fifty) are listed in `crossing` for
+// k_tree_top, which does the same from global memory: a search over the keys, and the pyramid of the
+// blocks' upper levels.
+//
+// All of it is independent per node, with the warps' lanes in step.  Former passes: a search over the
+// keys per node for range and split, leaf gather, pyramid, range unions and (NODES) the traversal nodes
+// (1.31M keys: 150 us with the nodes' 35, bound by dependent loads with 14 of 32 lanes active); now 97
+// us, with nodes 133.  Climbing from the leaves, the second child to arrive going on, took 82 us within
+// blocks (11 of 32 lanes) and 58 us across them (fences).
+constexpr int TREE_THREADS = 512;
+constexpr int TREE_LEVELS = 9;   // 2^9 gaps
+constexpr unsigned TOP_BLOCKS = 152 * 16;
+// start of the block pyramid's level l: 512, 128, 32, 8 and 2 boxes
+__host__ __device__ constexpr int tree_pyr(int l) { return l == 0 ? 0 : l == 1 ? 512 : l == 2 ? 640 : l == 3 ? 672 : 680; }
+constexpr int TREE_BOXES = 682;
+static_assert(TREE_THREADS == 1 << TREE_LEVELS, "gap table");
+
+// Length of the common prefix of two keys (code << 32 | primitive; delta, BVH.cuh:120-128): the
+// primitive word counts only when the codes are equal.  Keys are distinct.
+__device__ __forceinline__ int prefix_len(uint32_t ca, uint32_t oa, uint32_t cb, uint32_t ob)
 {
-    const uint32_t k = blockIdx.x * PYR_THREADS + threadIdx.x;
-    float4 mn, mx;
-    empty_box(mn, mx);
-    if (k < n) {
-        const uint32_t p = order[k];
-        mn = box_unsorted[2ull * p];
-        mx = box_unsorted[2ull * p + 1];
-        leaf_box[2ull * k] = mn;
-        leaf_box[2ull * k + 1] = mx;
-        if (keys) keys[k] = ((uint64_t)code[k] << 32) | p;
+    return ca != cb ? __clz(ca ^ cb) : 32 + __clz(oa ^ ob);
+}
+
+struct Box6 {
+    float v[6];
+    __device__ __forceinline__ void clear()
+    {
+#pragma unroll
+        for (int a = 0; a < 6; ++a) v[a] = a < 3 ? INFINITY : -INFINITY;
     }
-    if (levels) pyramid_up(mn, mx, n, levels, depth);
+    __device__ __forceinline__ void add(const Box6& b)
+    {
+#pragma unroll
+        for (int a = 0; a < 6; ++a) v[a] = a < 3 ? fminf(v[a], b.v[a]) : fmaxf(v[a], b.v[a]);
+    }
+};
+
+__device__ __forceinline__ Box6 box6(float4 mn, float4 mx) { return Box6{{mn.x, mn.y, mn.z, mx.x, mx.y, mx.z}}; }
+
+// Union of the block's boxes [lo, hi) from its pyramid in shared memory, as range_union.
+__device__ __forceinline__ Box6 block_union(const float (&pyr)[6][TREE_BOXES], int lo, int hi)
+{
+    Box6 b;
+    b.clear();
+    auto take = [&](int k) {
+#pragma unroll
+        for (int a = 0; a < 6; ++a) b.v[a] = a < 3 ? fminf(b.v[a], pyr[a][k]) : fmaxf(b.v[a], pyr[a][k]);
+    };
+#pragma unroll
+    for (int l = 0; l < 5; ++l) {
+        const int up = (lo + 3) & ~3, dn = hi & ~3;
+        if (l == 4 || up >= dn) {
+            for (int j = lo; j < hi; ++j) take(tree_pyr(l) + j);
+            break;
+        }
+        for (int j = lo; j < up; ++j) take(tree_pyr(l) + j);
+        for (int j = dn; j < hi; ++j) take(tree_pyr(l) + j);
+        lo = up >> 2;
+        hi = dn >> 2;
+    }
+    return b;
+}
+
+// Writes the node that splits behind key s and covers [first, last]; box_of(lo, hi) is the union of
+// leaf boxes lo .. hi - 1.
+template <bool NODES, typename BoxOf>
+__device__ __forceinline__ void store_node(int s, int first, int last, bool root, bool left, const BoxOf& box_of,
+                                           int2* __restrict__ child, int2* __restrict__ range,
+                                           float4* __restrict__ node_box, float4* __restrict__ nodes)
+{
+    const uint32_t i = root ? 0u : (uint32_t)(left ? last : first);
+    const int2 c = make_int2(first == s ? ~s : s, s + 1 == last ? ~(s + 1) : s + 1);
+    child[i] = c;
+    range[i] = make_int2(first, last);
+    Box6 u;
+    if (NODES) {   // layout: k_bvh2_nodes
+        u = box_of(first, s + 1);
+        const Box6 r = box_of(s + 1, last + 1);
+        nodes[4ull * i + 0] = make_float4(u.v[0], u.v[3], u.v[1], u.v[4]);
+        nodes[4ull * i + 1] = make_float4(r.v[0], r.v[3], r.v[1], r.v[4]);
+        nodes[4ull * i + 2] = make_float4(u.v[2], u.v[5], r.v[2], r.v[5]);
+        nodes[4ull * i + 3] = make_float4(__int_as_float(c.x), __int_as_float(c.y), 0.f, 0.f);
+        u.add(r);
+    } else {
+        u = box_of(first, last + 1);
+    }
+    node_box[2ull * i] = make_float4(u.v[0], u.v[1], u.v[2], 0.f);
+    node_box[2ull * i + 1] = make_float4(u.v[3], u.v[4], u.v[5], 0.f);
+}
+
+// up: pyramid levels above the leaves by 16, 64 and 256 boxes, back to back (n2, n3, n4 boxes).
+template <bool NODES>
+__global__ void __launch_bounds__(TREE_THREADS) k_tree(const uint32_t* __restrict__ code,
+                                                       const uint32_t* __restrict__ order, int n,
+                                                       const float4* __restrict__ box_unsorted,
+                                                       float4* __restrict__ leaf_box, uint64_t* __restrict__ keys,
+                                                       int8_t* __restrict__ gaps, uint32_t* __restrict__ crossing,
+                                                       uint32_t* n_crossing, float4* __restrict__ up,
+                                                       int2* __restrict__ child, int2* __restrict__ range,
+                                                       float4* __restrict__ node_box, float4* __restrict__ nodes)
+{
+    constexpr int T = TREE_THREADS;
+    // low[k][g] = the smallest of gaps g .. g + 2^k - 1; gap g lies between keys base + g - 1 and base + g
+    __shared__ int8_t low[TREE_LEVELS][T + 1];
+    __shared__ float pyr[6][TREE_BOXES];
+    const int t = threadIdx.x;
+    const int base = blockIdx.x * T, i = base + t;
+    int p = -1;   // the gap behind this thread's key
+    Box6 b;
+    b.clear();
+    if (i < n) {
+        const uint32_t c = code[i], o = order[i];
+        if (i + 1 < n) p = prefix_len(c, o, code[i + 1], order[i + 1]);
+        if (t == 0) low[0][0] = (int8_t)(i > 0 ? prefix_len(code[i - 1], order[i - 1], c, o) : -1);
+        const float4 mn = box_unsorted[2ull * o], mx = box_unsorted[2ull * o + 1];
+        leaf_box[2ull * i] = mn;
+        leaf_box[2ull * i + 1] = mx;
+        if (keys) keys[i] = ((uint64_t)c << 32) | o;
+        b = box6(mn, mx);
+        gaps[i] = (int8_t)p;
+    }
+    low[0][t + 1] = (int8_t)p;
+#pragma unroll
+    for (int a = 0; a < 6; ++a) pyr[a][t] = b.v[a];
+    __syncthreads();
+#pragma unroll
+    for (int k = 1; k < TREE_LEVELS; ++k) {
+        const int w = 1 << (k - 1);
+        for (int g = t; g + 2 * w <= T + 1; g += T) low[k][g] = min(low[k - 1][g], low[k - 1][g + w]);
+        if (k <= 4) {   // pyramid level k: T >> 2k boxes
+            const int m = T >> (2 * k);
+            if (t < m) {
+                Box6 u;
+                u.clear();
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int a = 0; a < 6; ++a)
+                        u.v[a] = a < 3 ? fminf(u.v[a], pyr[a][tree_pyr(k - 1) + 4 * t + j])
+                                       : fmaxf(u.v[a], pyr[a][tree_pyr(k - 1) + 4 * t + j]);
+#pragma unroll
+                for (int a = 0; a < 6; ++a) pyr[a][tree_pyr(k) + t] = u.v[a];
+                if (k >= 2) {
+                    const uint32_t n2 = ((uint32_t)n + 15) / 16, n3 = (n2 + 3) / 4, n4 = (n3 + 3) / 4;
+                    const uint32_t at = (uint32_t)blockIdx.x * m + t, count = k == 2 ? n2 : k == 3 ? n3 : n4,
+                                   from = k == 2 ? 0 : k == 3 ? n2 : n2 + n3;
+                    if (at < count)
+                        store_box(up, from + at, make_float4(u.v[0], u.v[1], u.v[2], 0.f),
+                                  make_float4(u.v[3], u.v[4], u.v[5], 0.f));
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (i + 1 >= n) return;
+    // nearest smaller gap on either side of gap g
+    const int g = t + 1;
+    int a = g, z = g;   // gaps a .. z are not smaller than p
+#pragma unroll
+    for (int k = TREE_LEVELS - 1; k >= 0; --k) {
+        const int w = 1 << k;
+        if (a - w >= 0 && low[k][a - w] >= p) a -= w;
+        if (z + w <= T && low[k][z + 1] >= p) z += w;
+    }
+    if (a == 0 || z == T) {
+        cg::coalesced_group cgp = cg::coalesced_threads();
+        uint32_t at = 0;
+        if (cgp.thread_rank() == 0) at = atomicAdd(n_crossing, (uint32_t)cgp.size());
+        crossing[cgp.shfl(at, 0) + cgp.thread_rank()] = (uint32_t)i;
+        return;
+    }
+    const int before = low[0][a - 1], behind = low[0][z + 1];
+    store_node<NODES>(
+        i, base + a - 1, base + z, before < 0 && behind < 0, behind > before,
+        [&](int lo, int hi) { return block_union(pyr, lo - base, hi - base); }, child, range, node_box, nodes);
+}
+
+// Union of leaf boxes [lo, hi) from the leaves, 16 at a time, and the levels above them.
+__device__ __forceinline__ Box6 wide_union(const float4* __restrict__ leaves, const float4* __restrict__ up, uint32_t n,
+                                           uint32_t lo, uint32_t hi)
+{
+    Box6 b;
+    b.clear();
+    const float4* a = leaves;
+    const float4* next = up;
+    uint32_t na = n;
+    for (uint32_t step = 16;; step = 4) {
+        const uint32_t up_lo = (lo + step - 1) & ~(step - 1), dn = hi & ~(step - 1);
+        if (up_lo >= dn) {
+#pragma unroll 4
+            for (uint32_t j = lo; j < hi; ++j) b.add(box6(a[2ull * j], a[2ull * j + 1]));
+            return b;
+        }
+#pragma unroll 4
+        for (uint32_t j = lo; j < up_lo; ++j) b.add(box6(a[2ull * j], a[2ull * j + 1]));
+#pragma unroll 4
+        for (uint32_t j = dn; j < hi; ++j) b.add(box6(a[2ull * j], a[2ull * j + 1]));
+        lo = up_lo / step;
+        hi = dn / step;
+        na = (na + step - 1) / step;
+        a = next;
+        next += 2ull * na;
+    }
+}
+
+template <bool NODES>
+__global__ void __launch_bounds__(64) k_tree_top(const uint32_t* __restrict__ code, const uint32_t* __restrict__ order,
+                                                 int n, const uint32_t* __restrict__ crossing,
+                                                 const uint32_t* __restrict__ n_crossing,
+                                                 const int8_t* __restrict__ gaps, const float4* __restrict__ leaf_box,
+                                                 const float4* __restrict__ up, int2* __restrict__ child,
+                                                 int2* __restrict__ range, float4* __restrict__ node_box,
+                                                 float4* __restrict__ nodes)
+{
+    const uint32_t count = *n_crossing;
+    for (uint32_t k = blockIdx.x * 64 + threadIdx.x; k < count; k += gridDim.x * 64) {
+        const int s = (int)crossing[k];
+        const uint32_t c = code[s], o = order[s];
+        const int p = gaps[s];
+        // both ends: the farthest keys that share p bits with key s, by doubling steps, then halving
+        // ones; the two searches step together
+        int lo = s, hi = s + 1;
+        int wl = 64, wh = 64;
+        bool gl = true, gh = true;   // still doubling
+        while (wl || wh) {
+            const int jl = lo - wl, jh = hi + wh;
+            const bool il = wl && wl <= lo, ih = wh && wh < n - hi;
+            const uint32_t cl = il ? code[jl] : 0u, ol = il ? order[jl] : 0u, ch = ih ? code[jh] : 0u,
+                           oh = ih ? order[jh] : 0u;
+            if (wl) {
+                if (il && prefix_len(cl, ol, c, o) >= p) {
+                    lo = jl;
+                    wl = gl ? (wl < 1 << 30 ? wl * 2 : wl) : wl / 2;
+                } else {
+                    gl = false;
+                    wl /= 2;
+                }
+            }
+            if (wh) {
+                if (ih && prefix_len(c, o, ch, oh) >= p) {
+                    hi = jh;
+                    wh = gh ? (wh < 1 << 30 ? wh * 2 : wh) : wh / 2;
+                } else {
+                    gh = false;
+                    wh /= 2;
+                }
+            }
+        }
+        const int before = lo > 0 ? gaps[lo - 1] : -1, behind = gaps[hi];
+        store_node<NODES>(
+            s, lo, hi, before < 0 && behind < 0, behind > before,
+            [&](int x, int y) { return wide_union(leaf_box, up, (uint32_t)n, (uint32_t)x, (uint32_t)y); }, child, range,
+            node_box, nodes);
+    }
 }
 
 // Union of leaf boxes [lo, hi) (exclusive hi) from the pyramid: at each level the partial groups
@@ -880,8 +1083,16 @@ __global__ void k_leaf_records(const uint32_t* __restrict__ order, uint32_t n, u
 
 inline unsigned blocks_for(uint64_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
 
+// Threads of a sort block (4 or 8 keys each).  A tile adds up the counts of the tiles before it that
+// run beside it, so there should be about as many tiles as SMs; below that, small tiles, since a pass
+// lasts as long as one tile.
+int sort_threads(uint32_t n) { return n <= 1u << 15 ? 256 : n <= 1u << 19 ? 512 : 1024; }
+uint32_t sort_tile(uint32_t n) { return (uint32_t)sort_threads(n) * (sort_threads(n) == 256 ? 4u : 8u); }
+// Words of the sort's chains hold two flag bits beside a count of up to n.
+size_t chain_word(uint32_t n) { return n < 1u << 30 ? 4 : 8; }
+
 struct ScratchLayout {
-    size_t code0, code1, val1, counts, totals, box_unsorted, levels, total;
+    size_t code0, code1, val1, totals, tickets, state, sort_clear, box_unsorted, levels, total;
     uint32_t num_tiles;
     int level_count;   // pyramid levels above the leaves (0 for a single leaf)
 };
@@ -892,49 +1103,66 @@ ScratchLayout layout_for(uint32_t n)
     std::memset(&L, 0, sizeof L);
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 256); return o; };
-    L.num_tiles = (n + RS_TILE - 1) / RS_TILE;
+    const uint32_t tile = sort_tile(n);
+    L.num_tiles = (uint32_t)(((uint64_t)n + tile - 1) / tile);
     L.code0 = take((size_t)n * 4);
-    // The sort's second key/value buffers and its tile counts are dead once the sort has ended;
-    // the box pyramid, built after it, takes their place.
+    // The sort's second buffers and its chains are dead once the tree is built; a refit's box pyramid
+    // takes their place.
     const size_t n4 = align_up((size_t)n * 4, 256);
-    const size_t counts = align_up((size_t)RS_BINS * std::max(1u, L.num_tiles) * 4, 256);
-    const size_t sort_bytes = 2 * n4 + counts + (size_t)RS_PASSES * RS_BINS * 4;
+    const size_t totals = RS_PASSES * RS_BINS * 4;
+    L.sort_clear = totals + 256 + (size_t)RS_PASSES * L.num_tiles * RS_BINS * chain_word(n);
+    const size_t sort_bytes = 2 * n4 + L.sort_clear;
     size_t lv_boxes = 0;
     for (uint32_t m = n; m > 1;) {
-        m = (m + 3) / 4;
+        m = (uint32_t)(((uint64_t)m + 3) / 4);
         lv_boxes += m;
         L.level_count++;
     }
     const size_t shared = take(std::max(sort_bytes, lv_boxes * 32));
     L.code1 = shared;
     L.val1 = shared + n4;
-    L.counts = shared + 2 * n4;
-    L.totals = shared + 2 * n4 + counts;
+    L.totals = shared + 2 * n4;   // totals, tickets and chains are cleared together
+    L.tickets = L.totals + totals;
+    L.state = L.tickets + 256;
     L.levels = shared;
     L.box_unsorted = take((size_t)n * 32);
     L.total = off;
     return L;
 }
 
-// The pyramid above the sorted leaf boxes, from level `from` (1: the leaves' first level is
-// already in the scratch), then the node boxes.
+template <int THREADS, int ITEMS, typename Word>
+cpt_status sort_passes(uint32_t n, const ScratchLayout& SL, char* base, uint32_t* code0, uint32_t* code1,
+                       uint32_t* val0, uint32_t* val1, cudaStream_t stream)
+{
+    const uint32_t* totals = (const uint32_t*)(base + SL.totals);
+    uint32_t* tickets = (uint32_t*)(base + SL.tickets);
+    Word* state = (Word*)(base + SL.state);
+    const size_t per_pass = (size_t)SL.num_tiles * RS_BINS;
+    const int smem = (int)sizeof(SortSmem<THREADS, ITEMS, Word>);
+    for (int p = 0; p < RS_PASSES; ++p) {
+        uint32_t *ki = p & 1 ? code1 : code0, *vi = p & 1 ? val1 : val0, *ko = p & 1 ? code0 : code1,
+                 *vo = p & 1 ? val0 : val1;
+        const auto k = p == 0 ? k_sort_digit<THREADS, ITEMS, Word, true> : k_sort_digit<THREADS, ITEMS, Word, false>;
+        if (smem > 48 << 10) CPT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        k<<<SL.num_tiles, THREADS, smem, stream>>>(ki, vi, ko, vo, n, RS_BITS * p, totals + p * RS_BINS,
+                                                   state + p * per_pass, tickets + p);
+    }
+    CPT_CUDA(cudaGetLastError());
+    add_launches(RS_PASSES);
+    return CPT_OK;
+}
+
+// The pyramid above the sorted leaf boxes, then the node boxes.
 cpt_status refit_from_leaves(uint32_t n, const ScratchLayout& SL, char* base, const int2* range, float4* node_box,
-                             const float4* leaf_box, cudaStream_t stream, int from = 0)
+                             const float4* leaf_box, cudaStream_t stream)
 {
     if (n < 2) return CPT_OK;
     float4* levels = (float4*)(base + SL.levels);
-    // walk to level `from`
     const float4* in = leaf_box;
     float4* out = levels;
     uint32_t m = n;
-    for (int l = 0; l < from; ++l) {
-        const uint32_t up = (m + 3) / 4;
-        in = out;
-        out += 2ull * up;
-        m = up;
-    }
     int launches = 1;
-    for (int l = from; l < SL.level_count; l += 4) {
+    for (int l = 0; l < SL.level_count; l += 4) {
         const int depth = std::min(4, SL.level_count - l);
         k_pyramid<<<blocks_for(m, PYR_THREADS), PYR_THREADS, 0, stream>>>(in, m, out, depth);
         launches++;
@@ -972,18 +1200,12 @@ cpt_status lbvh_build(uint32_t n_extra, const double* extra_centroid, const floa
     if (!scratch || scratch_bytes < SL.total || ((uintptr_t)scratch & 255u))
         return fail(CPT_ERR_INVALID_ARGUMENT, "lbvh_build: scratch too small or not 256-byte aligned");
     char* base = (char*)scratch;
-    // Keys and values ping-pong between (code0, val0 = out.order) and (code1, val1); k_prep fills
-    // the pair that makes the last pass end in out.order.
+    // Keys and values ping-pong between (code0, val0 = out.order) and (code1, val1); an even number
+    // of passes ends where it began.
     uint32_t* code0 = (uint32_t*)(base + SL.code0);
     uint32_t* code1 = (uint32_t*)(base + SL.code1);
     uint32_t* val0 = out.order;
     uint32_t* val1 = (uint32_t*)(base + SL.val1);
-    constexpr bool odd = (RS_PASSES & 1) != 0;
-    uint32_t* kin = odd ? code1 : code0;
-    uint32_t* vin = odd ? val1 : val0;
-    uint32_t* kout = odd ? code0 : code1;
-    uint32_t* vout = odd ? val0 : val1;
-    uint32_t* counts = (uint32_t*)(base + SL.counts);
     uint32_t* totals = (uint32_t*)(base + SL.totals);
     float4* box_unsorted = (float4*)(base + SL.box_unsorted);
 
@@ -1008,50 +1230,66 @@ cpt_status lbvh_build(uint32_t n_extra, const double* extra_centroid, const floa
         return m;
     };
     const MortonAxis ax = axis(smin.x, smax.x), ay = axis(smin.y, smax.y), az = axis(smin.z, smax.z);
+    CPT_CUDA(cudaMemsetAsync(totals, 0, SL.sort_clear, stream));
+    const unsigned prep_grid = std::min(blocks_for(n, PREP_THREADS), PREP_BLOCKS);
     if (tri_f64)
-        k_prep<double><<<blocks_for(n, 256), 256, 0, stream>>>(n_extra, extra_centroid, extra_box, n_tri, tri_f64, ax,
-                                                               ay, az, kin, vin, box_unsorted);
+        k_prep<double><<<prep_grid, PREP_THREADS, 0, stream>>>(n_extra, extra_centroid, extra_box, n_tri, tri_f64, ax,
+                                                               ay, az, code0, box_unsorted, totals);
     else
-        k_prep<float><<<blocks_for(n, 256), 256, 0, stream>>>(n_extra, extra_centroid, extra_box, n_tri, tri_f32, ax,
-                                                              ay, az, kin, vin, box_unsorted);
+        k_prep<float><<<prep_grid, PREP_THREADS, 0, stream>>>(n_extra, extra_centroid, extra_box, n_tri, tri_f32, ax,
+                                                              ay, az, code0, box_unsorted, totals);
     CPT_CUDA(cudaGetLastError());
     add_launches(1);
     if (stages) CPT_CUDA(cudaEventRecord(stages[1], stream));
 
-    // Radix sort: RS_PASSES passes of RS_BITS bits, ending in code0/val0 (= out.order).
-    CPT_CUDA(cudaMemsetAsync(totals, 0, RS_PASSES * RS_BINS * 4, stream));
-    k_digit_totals<<<std::min(blocks_for(n, 256), 1024u), 256, 0, stream>>>(kin, n, totals);
-    CPT_CUDA(cudaFuncSetAttribute(k_radix_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(ScatterSmem)));
-    CPT_CUDA(cudaFuncSetAttribute(k_radix_scatter, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                  cudaSharedmemCarveoutMaxShared));
-    CPT_CUDA(cudaFuncSetAttribute(k_radix_hist, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                  cudaSharedmemCarveoutMaxShared));
-    for (int p = 0; p < RS_PASSES; ++p) {
-        k_radix_hist<<<SL.num_tiles, RS_THREADS, 0, stream>>>(kin, n, RS_BITS * p, counts, SL.num_tiles);
-        k_radix_scan<<<RS_BINS, 256, 0, stream>>>(counts, SL.num_tiles, totals + p * RS_BINS);
-        k_radix_scatter<<<SL.num_tiles, RS_THREADS, sizeof(ScatterSmem), stream>>>(kin, vin, kout, vout, n, RS_BITS * p,
-                                                                                  counts, SL.num_tiles);
-        std::swap(kin, kout);
-        std::swap(vin, vout);
-    }
-    CPT_CUDA(cudaGetLastError());
-    add_launches(1 + 3 * RS_PASSES);
+    const auto sort = chain_word(n) == 8        ? sort_passes<1024, 8, unsigned long long>
+                      : sort_threads(n) == 1024 ? sort_passes<1024, 8, uint32_t>
+                      : sort_threads(n) == 512  ? sort_passes<512, 8, uint32_t>
+                                                : sort_passes<256, 4, uint32_t>;
+    const cpt_status st = sort(n, SL, base, code0, code1, val0, val1, stream);
+    if (st != CPT_OK) return st;
     if (stages) CPT_CUDA(cudaEventRecord(stages[2], stream));
 
-    // Emission + sorted leaf boxes.
-    if (n > 1) k_emit<<<blocks_for(n - 1, 256), 256, 0, stream>>>(kin, vin, (int)n, out.child, out.range);
-    const int depth = std::min(4, SL.level_count);
-    float4* levels = depth > 0 ? (float4*)(base + SL.levels) : nullptr;
-    k_leaves<<<blocks_for(n, PYR_THREADS), PYR_THREADS, 0, stream>>>(kin, vin, n, box_unsorted, out.leaf_box,
-                                                                    out.keys, levels, depth);
+    // Hierarchy, leaf and node boxes.  The sort's second buffers are free: code1 takes the list of
+    // crossing gaps, val1 the upper pyramid levels (8/3 bytes a primitive), the chains' room the gaps.
+    int8_t* gaps = (int8_t*)(base + SL.state);
+    uint32_t* n_crossing = (uint32_t*)(base + SL.tickets) + RS_PASSES;
+    float4* up = (float4*)val1;
+    const unsigned tree_grid = blocks_for(n, TREE_THREADS), top_grid = std::min(blocks_for(n, 64), TOP_BLOCKS);
+    const auto tree = out.nodes ? k_tree<true> : k_tree<false>;
+    tree<<<tree_grid, TREE_THREADS, 0, stream>>>(code0, val0, (int)n, box_unsorted, out.leaf_box, out.keys, gaps, code1,
+                                                 n_crossing, up, out.child, out.range, out.node_box, out.nodes);
+    if (n > TREE_THREADS) {   // nodes reach across blocks: the rest of the pyramid, then those nodes
+        const uint32_t n2 = (n + 15) / 16, n3 = (n2 + 3) / 4;
+        const float4* in = up + 2ull * (n2 + n3);
+        uint32_t m = (n3 + 3) / 4;
+        float4* next = up + 2ull * (n2 + n3 + m);
+        while (m > 1) {
+            int depth = 0;
+            uint32_t top = m;
+            float4* after = next;
+            const float4* last = in;
+            while (depth < 4 && top > 1) {
+                top = (top + 3) / 4;
+                last = after;
+                after += 2ull * top;
+                depth++;
+            }
+            k_pyramid<<<blocks_for(m, PYR_THREADS), PYR_THREADS, 0, stream>>>(in, m, next, depth);
+            add_launches(1);
+            in = last;
+            next = after;
+            m = top;
+        }
+        const auto rest = out.nodes ? k_tree_top<true> : k_tree_top<false>;
+        rest<<<top_grid, 64, 0, stream>>>(code0, val0, (int)n, code1, n_crossing, gaps, out.leaf_box, up, out.child,
+                                          out.range, out.node_box, out.nodes);
+        add_launches(1);
+    }
     CPT_CUDA(cudaGetLastError());
-    add_launches((n > 1 ? 1 : 0) + 1);
+    add_launches(1);
     if (stages) CPT_CUDA(cudaEventRecord(stages[3], stream));
-
-    cpt_status st = refit_from_leaves(n, SL, base, out.range, out.node_box, out.leaf_box, stream, depth);
-    if (st != CPT_OK) return st;
-    if (stages) CPT_CUDA(cudaEventRecord(stages[4], stream));
+    if (stages) CPT_CUDA(cudaEventRecord(stages[4], stream));   // boxes came with the hierarchy: no refit
     return CPT_OK;
 }
 
@@ -1116,6 +1354,7 @@ CPT_EXPORT cpt_status cpt_lbvh_build_device(uint32_t num_extra, const double* ex
     b.range = (int2*)out_node_range;
     b.node_box = (float4*)out_node_boxes;
     b.leaf_box = (float4*)out_leaf_boxes;
+    b.nodes = nullptr;
     return cpt::lbvh_build(num_extra, extra_centroids, (const float4*)extra_boxes, num_tri, tri_vertices, nullptr,
                            scene_min, scene_max, b, scratch, scratch_bytes, (cudaStream_t)stream, nullptr);
 }

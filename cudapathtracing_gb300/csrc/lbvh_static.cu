@@ -129,8 +129,9 @@ CPT_EXPORT cpt_status cpt_lbvh_build_device_static(uint32_t num_extra, const dou
     b.range = (int2*)out_node_range;
     b.node_box = (float4*)out_node_boxes;
     b.leaf_box = (float4*)out_leaf_boxes;
-    // The build clears the digit totals it accumulates into; every other scratch word is written
-    // before it is read, so the previous call's contents do no harm.
+    b.nodes = nullptr;
+    // The build clears the sort's counters and chains; every other scratch word is written before it
+    // is read, so the previous call's contents do no harm.
     return cpt::lbvh_build(num_extra, extra_centroids, (const float4*)extra_boxes, num_tri, tri_vertices, nullptr,
                            scene_min, scene_max, b, scratch, kStaticScratchBytes, (cudaStream_t)stream, nullptr);
 }
