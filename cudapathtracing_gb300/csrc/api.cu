@@ -46,7 +46,7 @@ using namespace cpt;
 struct HostWords {
     unsigned long long rays;
     int err;
-    int cnt[16];
+    int cnt[WIDE_HOST_WORDS];
 };
 
 struct cpt_context {
@@ -78,10 +78,6 @@ constexpr uint64_t STAGED_RAYS = 16384;
 namespace cpt {
 cpt_status wavefront_grids(int sm_count, int block_trace, int block_shade, int short_entries, int* grid_trace,
                            int* grid_trace_wide, int* grid_shade, int* grid_paths);
-size_t wide_scratch_bytes(uint32_t n);
-cpt_status build_wide(uint32_t n, const int2* child, const float4* node_box, const float4* leaf_box,
-                      const uint32_t* order, float4* wide, void* scratch, size_t scratch_bytes, cudaStream_t stream,
-                      uint32_t* num_wide, const uint32_t** wide_order);
 }
 
 struct cpt_scene {
@@ -453,57 +449,6 @@ SceneView view_of(const cpt_scene* s)
     return v;
 }
 
-// Binary traversal nodes (either format), allocated on first use.
-cpt_status need_nodes(cpt_scene* s)
-{
-    return s->nodes || s->n < 2 ? CPT_OK : dalloc(&s->nodes, 4 * (size_t)(s->n - 1));
-}
-
-// Traversal layout for the context's BVH width: the compressed 8-wide BVH (collapse in wide.cu,
-// using the LBVH scratch for its task queues) or the BVH2 node array; leaf records in the
-// matching order.  Buffers are allocated on first use.
-// `nodes_ready`: the build has written the 64-byte binary nodes along with the hierarchy.
-cpt_status make_layout(cpt_scene* s, cudaStream_t stream, uint32_t* num_wide, bool nodes_ready)
-{
-    uint32_t n = s->n;
-    uint32_t ni = n > 1 ? n - 1 : 0;
-    int width = s->ctx->bvh_width;
-    if (width == 8 && n > 1) {
-        if (!s->wide) {
-            cpt_status st = dalloc(&s->wide, CPT_WIDE_F4 * (size_t)ni);
-            if (st != CPT_OK) return st;
-        }
-        if (wide_scratch_bytes(n) > s->scratch_bytes) return fail(CPT_ERR_INVALID_ARGUMENT, "wide scratch too small");
-        s->width = 8;
-        const uint32_t* wide_order = nullptr;   // primitives of the leaves in the wide layout's order
-        cpt_status st = build_wide(n, s->child, s->node_box, s->leaf_box, s->order, s->wide, s->scratch,
-                                   s->scratch_bytes, stream, num_wide, &wide_order);
-        if (st != CPT_OK) return st;
-        return build_trace_layout(n, s->n_lights, s->n_spheres, s->child, s->node_box, s->leaf_box, wide_order,
-                                  s->tri_f32, s->tri_f64, s->spheres, nullptr, s->leaf_rec, stream);
-    }
-    cpt_status st = need_nodes(s);
-    if (st != CPT_OK) return st;
-    s->width = 2;
-    s->node_q = s->ctx->bvh2_compressed;
-    if (num_wide) *num_wide = 0;
-    return build_trace_layout(n, s->n_lights, s->n_spheres, s->child, s->node_box, s->leaf_box, s->order, s->tri_f32,
-                              s->tri_f64, s->spheres, nodes_ready ? nullptr : s->nodes, s->leaf_rec, stream, s->node_q);
-}
-
-LbvhBuffers buffers_of(cpt_scene* s)
-{
-    LbvhBuffers b;
-    b.keys = s->keys;
-    b.order = s->order;
-    b.child = s->child;
-    b.range = s->range;
-    b.node_box = s->node_box;
-    b.leaf_box = s->leaf_box;
-    b.nodes = nullptr;
-    return b;
-}
-
 // The context's workspace pool, made by the first call that needs it.
 cpt_status need_pool(cpt_context* c)
 {
@@ -551,6 +496,58 @@ cpt_status need_host(cpt_context* c)
         cpt_status _s = (call);             \
         if (_s != CPT_OK) return _s;        \
     } while (0)
+
+// Binary traversal nodes (either format), allocated on first use.
+cpt_status need_nodes(cpt_scene* s)
+{
+    return s->nodes || s->n < 2 ? CPT_OK : dalloc(&s->nodes, 4 * (size_t)(s->n - 1));
+}
+
+// Traversal layout for the context's BVH width: the compressed 8-wide BVH (collapse in wide.cu,
+// using the LBVH scratch for its task queues) or the BVH2 node array; leaf records in the
+// matching order.  Buffers are allocated on first use.
+// `nodes_ready`: the build has written the 64-byte binary nodes along with the hierarchy.
+cpt_status make_layout(cpt_scene* s, cudaStream_t stream, uint32_t* num_wide, bool nodes_ready)
+{
+    uint32_t n = s->n;
+    uint32_t ni = n > 1 ? n - 1 : 0;
+    int width = s->ctx->bvh_width;
+    if (width == 8 && n > 1) {
+        if (!s->wide) {
+            cpt_status st = dalloc(&s->wide, CPT_WIDE_F4 * (size_t)ni);
+            if (st != CPT_OK) return st;
+        }
+        if (wide_scratch_bytes(n) > s->scratch_bytes) return fail(CPT_ERR_INVALID_ARGUMENT, "wide scratch too small");
+        s->width = 8;
+        CPT_NEED(need_host(s->ctx));
+        return build_wide(n, s->child, s->node_box, s->leaf_box, s->order, s->wide, s->scratch, s->scratch_bytes, stream,
+                          num_wide, s->ctx->host->cnt, [&](const uint32_t* order, const uint32_t* n_ready) {
+                              return build_trace_layout(n, s->n_lights, s->n_spheres, s->child, s->node_box,
+                                                        s->leaf_box, order, s->tri_f32, s->tri_f64, s->spheres,
+                                                        nullptr, s->leaf_rec, stream, false, n_ready);
+                          });
+    }
+    cpt_status st = need_nodes(s);
+    if (st != CPT_OK) return st;
+    s->width = 2;
+    s->node_q = s->ctx->bvh2_compressed;
+    if (num_wide) *num_wide = 0;
+    return build_trace_layout(n, s->n_lights, s->n_spheres, s->child, s->node_box, s->leaf_box, s->order, s->tri_f32,
+                              s->tri_f64, s->spheres, nodes_ready ? nullptr : s->nodes, s->leaf_rec, stream, s->node_q);
+}
+
+LbvhBuffers buffers_of(cpt_scene* s)
+{
+    LbvhBuffers b;
+    b.keys = s->keys;
+    b.order = s->order;
+    b.child = s->child;
+    b.range = s->range;
+    b.node_box = s->node_box;
+    b.leaf_box = s->leaf_box;
+    b.nodes = nullptr;
+    return b;
+}
 
 // Reads and clears the device error word (synchronises the stream).
 cpt_status check_device_error(cpt_scene* s, cudaStream_t stream)

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <functional>
 #include <string>
 
 #include "cpt.h"
@@ -60,11 +61,21 @@ cpt_status lbvh_leaf_boxes(uint32_t n_extra, const float4* extra_box, uint32_t n
 
 // ---- traversal layout (lbvh.cu)
 // BVH2 nodes (4 float4 per internal node, or 2 when compressed: 8-bit quantised child boxes) and
-// leaf records (3 float4 per leaf).
+// leaf records (3 float4 per leaf; only the first *n_ready when it is given).
 cpt_status build_trace_layout(uint32_t n, uint32_t n_lights, uint32_t n_spheres, const int2* child,
                               const float4* node_box, const float4* leaf_box, const uint32_t* order,
                               const float* tri_f32, const double* tri_f64, const float4* spheres, float4* nodes,
-                              float4* leaf_rec, cudaStream_t stream, bool compressed = false);
+                              float4* leaf_rec, cudaStream_t stream, bool compressed = false,
+                              const uint32_t* n_ready = nullptr);
+
+// ---- 8-wide layout (wide.cu).  host_words: pinned, WIDE_HOST_WORDS ints.  leaf_records(order, n_ready)
+// queues the leaf records in the wide layout's order, of which the first *n_ready are known.
+constexpr int WIDE_HOST_WORDS = 160;
+using LeafRecords = std::function<cpt_status(const uint32_t* order, const uint32_t* n_ready)>;
+size_t wide_scratch_bytes(uint32_t n);
+cpt_status build_wide(uint32_t n, const int2* child, const float4* node_box, const float4* leaf_box,
+                      const uint32_t* order, float4* wide, void* scratch, size_t scratch_bytes, cudaStream_t stream,
+                      uint32_t* num_wide, int* host_words, const LeafRecords& leaf_records);
 
 // ---- trace / render launchers (trace.cu, render.cu)
 // resident: blocks of the trace kernels (binary, 8-wide) that fit the device at once.

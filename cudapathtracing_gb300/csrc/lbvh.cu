@@ -1048,10 +1048,10 @@ __device__ __forceinline__ float edge32(float b, float a)
 template <typename VT>
 __global__ void k_leaf_records(const uint32_t* __restrict__ order, uint32_t n, uint32_t n_lights, uint32_t n_spheres,
                                const VT* __restrict__ tri_v, const float4* __restrict__ spheres,
-                               float4* __restrict__ rec)
+                               const uint32_t* __restrict__ n_ready, float4* __restrict__ rec)
 {
     uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
+    if (k >= n || (n_ready && k >= *n_ready)) return;
     uint32_t p = order[k];
     float4 r0, r1, r2 = make_float4(0.f, 0.f, 0.f, 0.f);
     if (p < n_lights) {
@@ -1317,7 +1317,8 @@ cpt_status lbvh_refit(uint32_t n, const LbvhBuffers& out, void* scratch, size_t 
 cpt_status build_trace_layout(uint32_t n, uint32_t n_lights, uint32_t n_spheres, const int2* child,
                               const float4* node_box, const float4* leaf_box, const uint32_t* order,
                               const float* tri_f32, const double* tri_f64, const float4* spheres, float4* nodes,
-                              float4* leaf_rec, cudaStream_t stream, bool compressed)
+                              float4* leaf_rec, cudaStream_t stream, bool compressed,
+                              const uint32_t* n_ready)
 {
     if (n == 0) return CPT_OK;
     if (n > 1 && nodes && compressed)
@@ -1326,10 +1327,10 @@ cpt_status build_trace_layout(uint32_t n, uint32_t n_lights, uint32_t n_spheres,
         k_bvh2_nodes<<<blocks_for(n - 1, 256), 256, 0, stream>>>(child, node_box, leaf_box, n - 1, nodes);
     if (tri_f64)
         k_leaf_records<double><<<blocks_for(n, 256), 256, 0, stream>>>(order, n, n_lights, n_spheres, tri_f64, spheres,
-                                                                       leaf_rec);
+                                                                       n_ready, leaf_rec);
     else
         k_leaf_records<float><<<blocks_for(n, 256), 256, 0, stream>>>(order, n, n_lights, n_spheres, tri_f32, spheres,
-                                                                      leaf_rec);
+                                                                      n_ready, leaf_rec);
     CPT_CUDA(cudaGetLastError());
     add_launches((n > 1 && nodes ? 1 : 0) + 1);
     return CPT_OK;

@@ -54,14 +54,34 @@ __device__ __forceinline__ void ref_box(int ref, const float4* node_box, const f
 
 // Level l: the wide nodes [base, base + n) with base = level_base[l], n = level_count[l]; wide node
 // w stands for binary node tasks[w].  Internal children get the next numbers in level l + 1, which
-// starts at base + n (one atomic per node reserves their consecutive block).  The candidate
-// children's references, boxes and areas stay in registers (every array is indexed with
-// compile-time indices only), so each box is read once: an expansion costs two dependent loads
-// (the expanded node's children, then their two boxes).
-constexpr int COLLAPSE_THREADS = 128;
+// starts at base + n.
+//
+// Eight lanes make a node, lane k holding candidate child k (reference, box, area): an expansion
+// costs one round of loads (the two new children's boxes and their own children), the choice of the
+// next one and of the next (child, slot) pair three shuffles.  A block makes COLLAPSE_NODES nodes at a
+// time, reserves their children's and leaves' numbers with one atomic each and writes the nodes out
+// together.  The levels are bound by the latency of that chain and, the large ones, by how many nodes
+// are in flight: with a thread a node (152 registers, 12 warps an SM, two atomics a node) the 1.31M-
+// primitive collapse took 390 us.
+constexpr int COLLAPSE_NODES = 32;
+constexpr int COLLAPSE_THREADS = 8 * COLLAPSE_NODES;
 constexpr int MAX_WIDE_LEVELS = 80;
 
-__global__ void __launch_bounds__(COLLAPSE_THREADS, 3) k_collapse_level(const int2* __restrict__ child,
+// (value, index) pair of the greatest value over the 8 lanes of a node, the lowest index on ties.
+__device__ __forceinline__ void max_of_8(float& v, int& k)
+{
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+        const float v2 = __shfl_xor_sync(0xffffffffu, v, o);
+        const int k2 = __shfl_xor_sync(0xffffffffu, k, o);
+        if (v2 > v || (v2 == v && k2 < k)) {
+            v = v2;
+            k = k2;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(COLLAPSE_THREADS) k_collapse_level(const int2* __restrict__ child,
                                                                      const float4* __restrict__ node_box,
                                                                      const float4* __restrict__ leaf_box,
                                                                      int* __restrict__ tasks,
@@ -72,144 +92,129 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS, 3) k_collapse_level(const in
                                                                      uint32_t* __restrict__ n_leaves,
                                                                      float4* __restrict__ wide)
 {
+    __shared__ float4 out[COLLAPSE_NODES][CPT_WIDE_F4];
+    __shared__ int sums[2][COLLAPSE_NODES + 1];   // internal children and leaves of the nodes, then their first numbers
     const int n = level_count[l];
     const int base = level_base[l];
     if (blockIdx.x == 0 && threadIdx.x == 0) level_base[l + 1] = base + n;
-    int* n_out = level_count + l + 1;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const int b = tasks[base + t];   // binary node
-        int refs[8];
-        float4 cmn[8], cmx[8];
-        float car[8];
+    const int k = threadIdx.x & 7, node = threadIdx.x >> 3, lane = threadIdx.x & 31, lane0 = lane & ~7;
+    for (int t0 = blockIdx.x * COLLAPSE_NODES; t0 < n; t0 += gridDim.x * COLLAPSE_NODES) {
+        const bool valid = t0 + node < n;
+        const int b = valid ? tasks[base + t0 + node] : 0;   // binary node
         const int2 c = child[b];
-        float4 nmn, nmx;
+        float4 nmn, nmx, mn, mx;
         ref_box(b, node_box, leaf_box, nmn, nmx);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            refs[k] = -1;
-            car[k] = -1.0f;
-        }
-        refs[0] = c.x;
-        refs[1] = c.y;
-        ref_box(c.x, node_box, leaf_box, cmn[0], cmx[0]);
-        ref_box(c.y, node_box, leaf_box, cmn[1], cmx[1]);
-        car[0] = area(cmn[0], cmx[0]);
-        car[1] = area(cmn[1], cmx[1]);
+        int ref = k == 0 ? c.x : c.y;
+        ref_box(ref, node_box, leaf_box, mn, mx);
+        int2 own = child[max(ref, 0)];   // the candidate's children, fetched with its box
+        float ar = area(mn, mx);
         int nr = 2;
         // Replace the internal child of largest area by its two children (the first such child in
         // candidate order on ties) until there are 8 children or only leaves remain.
-#pragma unroll
         for (int step = 0; step < 6; ++step) {
-            int best = -1, best_ref = 0;
-            float best_a = -1.0f;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                if (k < nr && refs[k] >= 0 && car[k] > best_a) {
-                    best_a = car[k];
-                    best = k;
-                    best_ref = refs[k];
-                }
-            }
-            if (best < 0) break;
-            const int2 cc = child[best_ref];
-            float4 amn, amx, bmn, bmx;
-            ref_box(cc.x, node_box, leaf_box, amn, amx);
-            ref_box(cc.y, node_box, leaf_box, bmn, bmx);
-            const float aa = area(amn, amx), ab = area(bmn, bmx);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                if (k == best) {
-                    refs[k] = cc.x;
-                    cmn[k] = amn;
-                    cmx[k] = amx;
-                    car[k] = aa;
-                } else if (k == nr) {
-                    refs[k] = cc.y;
-                    cmn[k] = bmn;
-                    cmx[k] = bmx;
-                    car[k] = ab;
-                }
+            float best_a = k < nr && ref >= 0 && ar > -1.0f ? ar : -1.0f;
+            int best = k;
+            max_of_8(best_a, best);
+            const int2 cc = make_int2(__shfl_sync(0xffffffffu, own.x, lane0 | best),
+                                      __shfl_sync(0xffffffffu, own.y, lane0 | best));
+            const bool more = valid && best_a > -1.0f;
+            if (!__any_sync(0xffffffffu, more)) break;
+            if (!more) continue;
+            if (k == best || k == nr) {
+                ref = k == best ? cc.x : cc.y;
+                ref_box(ref, node_box, leaf_box, mn, mx);
+                own = child[max(ref, 0)];
+                ar = area(mn, mx);
             }
             ++nr;
         }
-        const float cx = 0.5f * (nmn.x + nmx.x), cy = 0.5f * (nmn.y + nmx.y), cz = 0.5f * (nmn.z + nmx.z);
+        __syncwarp();
         // greedy slot assignment by direction: each round takes the (child, slot) pair of least cost
-        float dx[8], dy[8], dz[8];
-        int slot_of[8];
+        const float dx = 0.5f * (mn.x + mx.x) - 0.5f * (nmn.x + nmx.x), dy = 0.5f * (mn.y + mx.y) - 0.5f * (nmn.y + nmx.y),
+                    dz = 0.5f * (mn.z + mx.z) - 0.5f * (nmn.z + nmx.z);
+        float gain[8];   // minus the costs
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            dx[k] = 0.5f * (cmn[k].x + cmx[k].x) - cx;
-            dy[k] = 0.5f * (cmn[k].y + cmx[k].y) - cy;
-            dz[k] = 0.5f * (cmn[k].z + cmx[k].z) - cz;
-            slot_of[k] = -1;
-        }
+        for (int s = 0; s < 8; ++s) gain[s] = (s & 1 ? -dx : dx) + (s & 2 ? -dy : dy) + (s & 4 ? -dz : dz);
+        int slot = k < nr ? -1 : 8;   // 8: no child
         uint32_t used = 0;
-        for (int round = 0; round < nr; ++round) {
-            float best = INFINITY;
-            int bk = -1, bs = -1;
+        for (int round = 0; round < 8; ++round) {
+            float best = -INFINITY;
+            int bs = 8;
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                if (k >= nr || slot_of[k] >= 0) continue;
-#pragma unroll
-                for (int s = 0; s < 8; ++s) {
-                    if ((used >> s) & 1u) continue;
-                    float cost = -((s & 1 ? -dx[k] : dx[k]) + (s & 2 ? -dy[k] : dy[k]) + (s & 4 ? -dz[k] : dz[k]));
-                    if (cost < best) {
-                        best = cost;
-                        bk = k;
-                        bs = s;
-                    }
+            for (int s = 0; s < 8; ++s)
+                if (!((used >> s) & 1u) && gain[s] > best) {
+                    best = gain[s];
+                    bs = s;
                 }
+            int pair = slot < 0 ? k * 16 + bs : 255;
+            if (slot >= 0) best = -INFINITY;
+            max_of_8(best, pair);
+            const bool open = round < nr;
+            if (!__any_sync(0xffffffffu, open)) break;
+            // a child whose box has no finite centre takes the lowest free slot
+            if ((pair & 15) == 8) pair = (pair & ~15) | (__ffs(~used) - 1);
+            if (open) {
+                if (k == pair >> 4) slot = pair & 15;
+                used |= 1u << (pair & 15);
             }
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-                if (k == bk) slot_of[k] = bs;
-            used |= 1u << bs;
         }
+        const bool leaf = ref < 0, has = valid && slot < 8;
+        uint32_t masks = has ? (leaf ? 0x8000u : 0x80u) >> slot : 0u;   // slot s at bit 7 - s: internal | leaf << 8
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) masks |= __shfl_xor_sync(0xffffffffu, masks, o);
+        const uint32_t imask = masks & 0xFFu, lmask = masks >> 8;
         // Internal children take consecutive wide numbers and leaves consecutive records, both in
         // slot order: the child in slot s is number first + (children of its kind in slots below s).
-        uint32_t imask = 0, lmask = 0;   // slot s at bit 7 - s
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if (k < nr) (refs[k] >= 0 ? imask : lmask) |= 0x80u >> slot_of[k];
-        const int n_int = __popc(imask), n_leaf = __popc(lmask);
-        const int first_child = base + n + (n_int ? atomicAdd(n_out, n_int) : 0);
-        const uint32_t first_leaf = n_leaf ? atomicAdd(n_leaves, (uint32_t)n_leaf) : 0u;
-        const uint32_t ex = grid_exponent(nmn.x, nmx.x), ey = grid_exponent(nmn.y, nmx.y),
-                       ez = grid_exponent(nmn.z, nmx.z);
-        const float isx = inv_grid(ex), isy = inv_grid(ey), isz = inv_grid(ez);
-        uint32_t q[6][2];
-#pragma unroll
-        for (int a = 0; a < 6; ++a) q[a][0] = q[a][1] = 0;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            if (k >= nr) break;
-            const int s = slot_of[k];
-            if (refs[k] >= 0)
-                tasks[first_child + __popc(imask >> (8 - s))] = refs[k];
-            else
-                wide_order[first_leaf + __popc(lmask >> (8 - s))] = order[~refs[k]];
-            const uint32_t sh = (uint32_t)(s & 3) * 8u;
-            const uint32_t v[6] = {q_lo(cmn[k].x, nmn.x, isx) << sh, q_hi(cmx[k].x, nmn.x, isx) << sh,
-                                   q_lo(cmn[k].y, nmn.y, isy) << sh, q_hi(cmx[k].y, nmn.y, isy) << sh,
-                                   q_lo(cmn[k].z, nmn.z, isz) << sh, q_hi(cmx[k].z, nmn.z, isz) << sh};
-#pragma unroll
-            for (int a = 0; a < 6; ++a) {
-                if (s < 4)
-                    q[a][0] |= v[a];
-                else
-                    q[a][1] |= v[a];
-            }
+        if (k == 0) {
+            sums[0][node] = __popc(imask);
+            sums[1][node] = __popc(lmask);
         }
-        float4* dst = wide + CPT_WIDE_F4 * (size_t)(base + t);
-        dst[0] = make_float4(nmn.x, nmn.y, nmn.z, __uint_as_float(ex << 23));
-        dst[1] = make_float4(__uint_as_float(ey << 23), __uint_as_float(ez << 23), __int_as_float(first_child),
-                             __uint_as_float(first_leaf));
+        for (int j = threadIdx.x; j < COLLAPSE_NODES * CPT_WIDE_F4; j += COLLAPSE_THREADS)
+            (&out[0][0])[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncthreads();
+        if (threadIdx.x < 64) {   // warp w: exclusive sums of kind w, and the block's share of its numbers
+            const int w = threadIdx.x >> 5, own = sums[w][lane];
+            int x = own;
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
-            dst[2 + a] = make_float4(__int_as_float((int)q[2 * a][0]), __int_as_float((int)q[2 * a][1]),
-                                     __int_as_float((int)q[2 * a + 1][0]), __int_as_float((int)q[2 * a + 1][1]));
-        dst[5] = make_float4(__uint_as_float(imask | lmask << 8), 0.f, 0.f, 0.f);
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            int first = 0;
+            if (lane == 31 && x) first = w ? (int)atomicAdd(n_leaves, (uint32_t)x) : base + n + atomicAdd(level_count + l + 1, x);
+            first = __shfl_sync(0xffffffffu, first, 31);
+            sums[w][lane] = first + x - own;
+        }
+        __syncthreads();
+        const int first_child = sums[0][node], first_leaf = sums[1][node];
+        // the grid of axis a from lane a (its directed division is a long sequence)
+        const uint32_t e_own = grid_exponent(k == 0 ? nmn.x : k == 1 ? nmn.y : nmn.z, k == 0 ? nmx.x : k == 1 ? nmx.y : nmx.z);
+        const uint32_t ex = __shfl_sync(0xffffffffu, e_own, lane0), ey = __shfl_sync(0xffffffffu, e_own, lane0 | 1),
+                       ez = __shfl_sync(0xffffffffu, e_own, lane0 | 2);
+        if (has) {
+            const uint32_t below = 8 - slot;
+            if (leaf) wide_order[first_leaf + __popc(lmask >> below)] = order[~ref];
+            else tasks[first_child + __popc(imask >> below)] = ref;
+            const float isx = inv_grid(ex), isy = inv_grid(ey), isz = inv_grid(ez);
+            uint8_t* q = reinterpret_cast<uint8_t*>(&out[node][2]) + slot;
+            q[0] = (uint8_t)q_lo(mn.x, nmn.x, isx);
+            q[8] = (uint8_t)q_hi(mx.x, nmn.x, isx);
+            q[16] = (uint8_t)q_lo(mn.y, nmn.y, isy);
+            q[24] = (uint8_t)q_hi(mx.y, nmn.y, isy);
+            q[32] = (uint8_t)q_lo(mn.z, nmn.z, isz);
+            q[40] = (uint8_t)q_hi(mx.z, nmn.z, isz);
+        }
+        if (valid && k == 0) {
+            out[node][0] = make_float4(nmn.x, nmn.y, nmn.z, __uint_as_float(ex << 23));
+            out[node][1] = make_float4(__uint_as_float(ey << 23), __uint_as_float(ez << 23), __int_as_float(first_child),
+                                       __int_as_float(first_leaf));
+            out[node][5] = make_float4(__uint_as_float(masks), 0.f, 0.f, 0.f);
+        }
+        __syncthreads();
+        float4* dst = wide + CPT_WIDE_F4 * (size_t)(base + t0);
+        const int words = min(COLLAPSE_NODES, n - t0) * CPT_WIDE_F4;
+        for (int j = threadIdx.x; j < words; j += COLLAPSE_THREADS) dst[j] = (&out[0][0])[j];
+        __syncthreads();
     }
 }
 
@@ -236,7 +241,7 @@ size_t wide_scratch_bytes(uint32_t n)
 
 cpt_status build_wide(uint32_t n, const int2* child, const float4* node_box, const float4* leaf_box,
                       const uint32_t* order, float4* wide, void* scratch, size_t scratch_bytes, cudaStream_t stream,
-                      uint32_t* num_wide, const uint32_t** wide_order)
+                      uint32_t* num_wide, int* host_words, const LeafRecords& leaf_records)
 {
     if (n < 2) {
         if (num_wide) *num_wide = 0;
@@ -247,16 +252,17 @@ cpt_status build_wide(uint32_t n, const int2* child, const float4* node_box, con
     int* tasks = (int*)p;
     p += align_up((size_t)n * 4, 256);
     uint32_t* prims = (uint32_t*)p;
-    *wide_order = prims;
     p += align_up((size_t)n * 4, 256);
     int* level_count = (int*)p;
     int* level_base = level_count + MAX_WIDE_LEVELS;
     uint32_t* n_leaves = (uint32_t*)(level_base + MAX_WIDE_LEVELS);
     k_collapse_init<<<1, 128, 0, stream>>>(tasks, level_count, level_base, n_leaves);
     add_launches(1);
-    // A grid that is resident at once; each thread takes nodes of its level in turn.  The host
-    // looks at the level counts once every 16 levels (the wide tree of a few million primitives
-    // has about a dozen; a level whose count is zero returns at once).
+    // A grid that is resident at once; each block takes nodes of its level in turn.  The host looks at
+    // the level counts after a batch of levels (first log8(n) + 5, which meshes need: 9 of 81,920
+    // primitives, 11 of 1.31M; then 8 at a time; a level whose count is zero returns at once but costs
+    // its launch, 2.5 us), after queueing the leaf records of the leaves found so far, so that nothing
+    // waits for its look.
     // per device (the first 64 ordinals; others are queried on every call)
     static int resident_of[64] = {};
     int dev = 0;
@@ -269,24 +275,28 @@ cpt_status build_wide(uint32_t n, const int2* child, const float4* node_box, con
         resident = std::max(1, sms * std::max(1, per_sm));
         if (dev >= 0 && dev < 64) resident_of[dev] = resident;
     }
-    const unsigned grid = std::max(1u, std::min((n + COLLAPSE_THREADS - 1) / COLLAPSE_THREADS, (unsigned)resident));
-    int l = 0;
-    int hc[2] = {0, 0};
-    for (;;) {
-        const int first = l, stop = std::min(l + 16, MAX_WIDE_LEVELS - 1);
-        for (; l < stop; ++l)
+    int l = 0, batch = 5;
+    for (uint64_t m = 1; m < n; m *= 8) ++batch;
+    for (;; batch = 8) {
+        const int first = l, stop = std::min(l + batch, MAX_WIDE_LEVELS - 1);
+        for (; l < stop; ++l) {
+            // level l has at most 8^l nodes, and no more than there are binary nodes
+            const uint64_t most = std::min<uint64_t>(l < 10 ? 1ull << (3 * l) : n, n);
+            const unsigned grid = (unsigned)std::min<uint64_t>((most + COLLAPSE_NODES - 1) / COLLAPSE_NODES, (uint64_t)resident);
             k_collapse_level<<<grid, COLLAPSE_THREADS, 0, stream>>>(child, node_box, leaf_box, tasks, level_count,
                                                                     level_base, l, order, prims, n_leaves, wide);
+        }
         add_launches(stop - first);
         CPT_CUDA(cudaGetLastError());
+        cpt_status st = leaf_records(prims, n_leaves);
+        if (st != CPT_OK) return st;
         // level l: its count (wide nodes still to collapse) and base (= wide nodes written)
-        CPT_CUDA(cudaMemcpyAsync(&hc[0], level_count + l, sizeof(int), cudaMemcpyDeviceToHost, stream));
-        CPT_CUDA(cudaMemcpyAsync(&hc[1], level_base + l, sizeof(int), cudaMemcpyDeviceToHost, stream));
+        CPT_CUDA(cudaMemcpyAsync(host_words, level_count, 2 * MAX_WIDE_LEVELS * sizeof(int), cudaMemcpyDeviceToHost, stream));
         CPT_CUDA(cudaStreamSynchronize(stream));
-        if (hc[0] == 0 || l >= MAX_WIDE_LEVELS - 1) break;
+        if (host_words[l] == 0 || l >= MAX_WIDE_LEVELS - 1) break;
     }
-    if (hc[0] != 0) return fail(CPT_ERR_STACK_OVERFLOW, "build_wide: collapse did not finish");
-    if (num_wide) *num_wide = (uint32_t)hc[1];
+    if (host_words[l] != 0) return fail(CPT_ERR_STACK_OVERFLOW, "build_wide: collapse did not finish");
+    if (num_wide) *num_wide = (uint32_t)host_words[MAX_WIDE_LEVELS + l];
     return CPT_OK;
 }
 
