@@ -212,7 +212,14 @@ __device__ __forceinline__ uint32_t xor_bits(uint32_t v, uint32_t o)
 // scalar multiply-adds, 283 ms packed.  Measured and left out: prefetching the next node before the
 // leaf tests (+4 %), testing the three interval conditions by sign instead of min/max with tmin and
 // best (+2 %).
-template <Query Q, typename Stack64>
+//
+// LEAVES_FIRST tests a visit's leaves before it chooses the next node; the results are the same.
+// Walks with dynamic fetching choose the node first (2 to 4 % faster: a batch of eight renders
+// over 8-wide layouts 36.5 -> 35.0 ms).  A loop that traces one ray to its end
+// (trace_closest_wide) tests leaves first: the other way round, the lanes whose stack ran empty
+// parted from their warp before the leaf tests (4.6 of 32 lanes active), Cornell 400x400 37.5
+// instead of 13.5 ms.
+template <Query Q, typename Stack64, bool LEAVES_FIRST = false>
 struct WideWalk {
     float3 o, d, idir;
     float tmin, best;
@@ -302,6 +309,17 @@ struct WideWalk {
         const uint32_t hits = xor_bits(masks & ((~misses & 0xFFu) * 0x0101u), first ^ 7u);
         const uint32_t ihits = hits & 0xFFu;
         uint32_t lhits = (hits >> 8) & 0xFFu;
+        // Tests the hit leaves; true when an any-hit ray has its answer.
+        const auto leaves = [&]() -> bool {
+            const uint32_t leaf0 = __float_as_uint(f1.w), lmask = (masks >> 8) & 0xFFu;
+            while (lhits) {
+                const uint32_t slot = (uint32_t)(__ffs(lhits) - 1) ^ first;
+                lhits &= lhits - 1;
+                if (visit_leaf<Q>(s, (int)(leaf0 + __popc(lmask >> (8u - slot))), o, d, best, hit, skip, any)) return true;
+            }
+            return false;
+        };
+        if (LEAVES_FIRST && leaves()) return true;
         // Continue with the first hit internal child; the others stay on the stack as one group.
         bool done = false;
         uint64_t g = (uint64_t)__float_as_uint(f1.z) | ((uint64_t)(ihits | ((masks & 0xFFu) << 8)) << 32);
@@ -324,12 +342,7 @@ struct WideWalk {
                 }
             }
         }
-        const uint32_t leaf0 = __float_as_uint(f1.w), lmask = (masks >> 8) & 0xFFu;
-        while (lhits) {
-            const uint32_t slot = (uint32_t)(__ffs(lhits) - 1) ^ first;
-            lhits &= lhits - 1;
-            if (visit_leaf<Q>(s, (int)(leaf0 + __popc(lmask >> (8u - slot))), o, d, best, hit, skip, any)) return true;
-        }
+        if (!LEAVES_FIRST && leaves()) return true;
         return done;
     }
 };
@@ -368,7 +381,7 @@ template <bool ANY>
 __device__ __forceinline__ bool trace_closest_wide(const SceneView& s, float3 o, float3 d, float tmin, float tmax,
                                                    Hit& hit, int* err, int skip)
 {
-    WideWalk<ANY ? Q_ANY : Q_CLOSEST, LocalStack64> w;
+    WideWalk<ANY ? Q_ANY : Q_CLOSEST, LocalStack64, true> w;
     w.stack.init();
     w.start(o, d, tmin, tmax, skip);
     while (!w.step(s, err)) {}
