@@ -3,7 +3,7 @@
 // The collapse runs level by level from the root, one launch per level with no host round trip
 // in between (the level counts and bases live on the device).  Wide nodes are numbered compactly
 // in that breadth-first order: level l occupies [base_l, base_l + n_l), and the internal children of a node
-// are numbered consecutively (one atomic per node reserves their block in the next level), so the
+// are numbered consecutively (one atomic per block of nodes reserves their numbers), so the
 // reachable nodes fill [0, num_wide) with siblings side by side and the top levels packed together
 // (the hot part of the tree stays within a few megabytes).  Leaves stay in sorted Morton order in the
 // leaf records.  Each wide node stands for one binary node b; starting from b's two children,
