@@ -36,8 +36,9 @@ struct BilateralConsts {
 // One separable pass over `src`: the centre value and the neighbours come from the same image
 // (in the reference the centre is read from pic, which holds the same values as the pass input).
 //
-// A tap costs about 20 arithmetic instructions and one expf, and the pass is bound by issuing them
-// (DRAM: 0.02 ms of 0.08 a pass at 1080p), so everything else is shared: a thread filters four pixels
+// A tap costs about 20 arithmetic instructions and one expf, and the pass is bound by the multiply-add
+// pipe (72 % of its cycles busy, issue slots 66 %, DRAM 15 % at 1080p); a pixel a thread was bound by
+// issue slots (82 %).  So everything else is shared: a thread filters four pixels
 // that follow one another along the pass and takes each neighbour once for the four, and two pixels
 // share a packed multiply-add.  The horizontal pass keeps its row, one array per component, in shared
 // memory (four neighbours' component in one conflict-free 16-byte load); in the vertical pass lanes
