@@ -1086,7 +1086,8 @@ inline unsigned blocks_for(uint64_t n, unsigned t) { return (unsigned)((n + t - 
 // Threads of a sort block (4 or 8 keys each).  A tile adds up the counts of the tiles before it that
 // run beside it, so there should be about as many tiles as SMs; below that, small tiles, since a pass
 // lasts as long as one tile.
-int sort_threads(uint32_t n) { return n <= 1u << 15 ? 256 : n <= 1u << 19 ? 512 : 1024; }
+constexpr uint32_t SORT_SMALL = 1u << 15, SORT_MEDIUM = 1u << 19;
+int sort_threads(uint32_t n) { return n <= SORT_SMALL ? 256 : n <= SORT_MEDIUM ? 512 : 1024; }
 uint32_t sort_tile(uint32_t n) { return (uint32_t)sort_threads(n) * (sort_threads(n) == 256 ? 4u : 8u); }
 // Words of the sort's chains hold two flag bits beside a count of up to n.
 size_t chain_word(uint32_t n) { return n < 1u << 30 ? 4 : 8; }
@@ -1181,7 +1182,16 @@ cpt_status refit_from_leaves(uint32_t n, const ScratchLayout& SL, char* base, co
 
 }  // namespace
 
-size_t lbvh_scratch_bytes(uint32_t n) { return layout_for(std::max(n, 1u)).total; }
+// Scratch for n primitives holds every smaller build too: where the sort's tiles grow (sort_tile) the
+// chains shrink, so the largest build of each smaller tile size counts as well (32,768 primitives need
+// 1,577,216 bytes, 32,769 by themselves 1,530,112).
+size_t lbvh_scratch_bytes(uint32_t n)
+{
+    size_t bytes = layout_for(std::max(n, 1u)).total;
+    for (uint32_t last : {SORT_SMALL, SORT_MEDIUM})
+        if (n > last) bytes = std::max(bytes, layout_for(last).total);
+    return bytes;
+}
 
 cpt_status lbvh_build(uint32_t n_extra, const double* extra_centroid, const float4* extra_box, uint32_t n_tri,
                       const float* tri_f32, const double* tri_f64, const double smin_in[3], const double smax_in[3],

@@ -318,7 +318,8 @@ cpt_status cpt_lbvh_export(const cpt_scene* scene, uint64_t* keys, uint32_t* ord
  *   out_children[2*(N-1)]  (child A, child B) per internal node, leaf k encoded as ~k
  *   out_node_range[2*(N-1)] (first, last) sorted-leaf range of each internal node
  *   out_node_boxes[8*(N-1)], out_leaf_boxes[8*N]  min xyz, 0, max xyz, 0
- *   scratch: cpt_lbvh_scratch_bytes(N) bytes, 256-byte aligned; work is ordered on stream. */
+ *   scratch: cpt_lbvh_scratch_bytes(N) bytes, 256-byte aligned (enough for every smaller N too); work
+ *            is ordered on stream. */
 size_t cpt_lbvh_scratch_bytes(uint32_t num_prims);
 cpt_status cpt_lbvh_build_device(uint32_t num_extra, const double* extra_centroids, const float* extra_boxes,
                                  uint32_t num_tri, const float* tri_vertices, const double scene_min[3],
