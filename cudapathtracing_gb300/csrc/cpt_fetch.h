@@ -1,0 +1,35 @@
+// cpt_fetch.h — index arithmetic of the dynamic ray fetch (trace_items_walk, cpt_trace.cuh), which also
+// compiles as host C++.
+//
+// Warps take items 0 .. n - 1 from one counter, up to 32 at a time, each until it has seen the end.  The
+// counter therefore ends up to 32 per warp above n, and n may be as large as 2^31 - 2, so counter and
+// sums are unsigned: as ints they wrap to negative numbers, which pass for items.
+#pragma once
+#include <stdint.h>
+
+#ifdef __CUDACC__
+#define CPT_HD __host__ __device__ __forceinline__
+#else
+#define CPT_HD inline
+#endif
+
+namespace cpt {
+
+// Lanes of a warp that take items, when n (> 0) items are spread over `warps` warps.
+CPT_HD int spread_lanes(int n, int warps)
+{
+    const uint32_t lanes = ((uint32_t)n + (uint32_t)warps - 1u) / (uint32_t)warps;
+    return lanes < 32u ? (int)lanes : 32;
+}
+
+// Whether a warp that took `count` items from `base` on has seen the end.
+CPT_HD bool fetch_ends(uint32_t base, int count, int n) { return base + (uint32_t)count >= (uint32_t)n; }
+
+// The rank-th of them, or -1 past the end.
+CPT_HD int fetched_item(uint32_t base, int rank, int n)
+{
+    const uint32_t r = base + (uint32_t)rank;
+    return r < (uint32_t)n ? (int)r : -1;
+}
+
+}  // namespace cpt

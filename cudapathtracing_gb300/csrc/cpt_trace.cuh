@@ -8,6 +8,7 @@
 #pragma once
 
 #include "cpt_device.cuh"
+#include "cpt_fetch.h"
 
 namespace cpt {
 
@@ -574,23 +575,20 @@ __device__ __forceinline__ uint32_t trace_items_walk(const Views& views, int n, 
     bool exhausted = false;
     uint32_t rays = 0;
     int lanes = 32;   // of this warp that take items
-    if (SPREAD) {
-        const int warps = (int)(gridDim.x * (blockDim.x >> 5));
-        lanes = min(32, (n + warps - 1) / warps);
-    }
+    if (SPREAD) lanes = spread_lanes(n, (int)(gridDim.x * (blockDim.x >> 5)));
     for (;;) {
         const bool idle = item < 0 && (!SPREAD || lane < lanes);
         const uint32_t m = __ballot_sync(0xffffffffu, idle);
         // refill once at least CPT_REFILL lanes are idle (one atomic and one divergent ray load per
         // batch instead of per finished ray): 1 -> 8 lanes is +10 % on the 1080p render (16: same)
         if (__popc(m) >= (SPREAD ? min(CPT_REFILL, lanes) : CPT_REFILL) && !exhausted) {
-            int base = 0;
-            if (lane == 0) base = atomicAdd(fetch, __popc(m));
+            uint32_t base = 0;
+            if (lane == 0) base = (uint32_t)atomicAdd(fetch, __popc(m));
             base = __shfl_sync(0xffffffffu, base, 0);
-            if (base + __popc(m) >= n) exhausted = true;
+            if (fetch_ends(base, __popc(m), n)) exhausted = true;
             if (idle) {
-                const int r = base + __popc(m & lane_mask_lt());
-                if (r < n) {
+                const int r = fetched_item(base, __popc(m & lane_mask_lt()), n);
+                if (r >= 0) {
                     float3 o, d;
                     float tmn, tmx;
                     int skip = -1;
