@@ -608,6 +608,7 @@ CPT_EXPORT cpt_status cpt_context_create(int device, cpt_context** out)
     c->host = nullptr;
     c->staging = c->staging_dev = nullptr;
     c->trace_resident[0] = c->trace_resident[1] = 0;
+    std::memset(c->time, 0, sizeof c->time);
     *out = c;
     return CPT_OK;
 }
@@ -685,8 +686,13 @@ CPT_EXPORT cpt_status cpt_filter_bilateral(cpt_context* ctx, const float* rgb, c
     if (params) p = *params;
     if (rgb == out) return fail(CPT_ERR_INVALID_ARGUMENT, "cpt_filter_bilateral: out must not alias rgb");
     CPT_CUDA(cudaSetDevice(ctx->device));
-    CPT_NEED(need_pool(ctx));
-    return filter_bilateral(rgb, gbuf, out, width, height, p, (cudaStream_t)stream, ctx->pool);
+    // Captured into a graph, the filter's buffer is an allocation node of the graph's own, from the
+    // device's default pool (the context's may not be made during a capture).
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CPT_CUDA(cudaStreamIsCapturing((cudaStream_t)stream, &capture));
+    if (capture == cudaStreamCaptureStatusNone) CPT_NEED(need_pool(ctx));
+    return filter_bilateral(rgb, gbuf, out, width, height, p, (cudaStream_t)stream,
+                            capture == cudaStreamCaptureStatusNone ? ctx->pool : nullptr);
 }
 
 CPT_EXPORT cpt_status cpt_filter_temporal(cpt_context* ctx, float* rgb, const float* prev_rgb, const float* gbuf,
@@ -1064,8 +1070,11 @@ CPT_EXPORT cpt_status cpt_render(cpt_scene* s, const cpt_render_params* p, const
     if (r0 < 0 || r1 > H || r0 > r1) return fail(CPT_ERR_INVALID_ARGUMENT, "cpt_render: bad row range");
     cudaStream_t stream = (cudaStream_t)stream_;
     CPT_CUDA(cudaSetDevice(s->ctx->device));
-    CPT_NEED(need_pool(s->ctx));
-    CPT_NEED(need_host(s->ctx));
+    // A megakernel render into device buffers without statistics only queues work, and may be captured:
+    // it needs neither (their first use allocates, which a capture does not allow).
+    const bool wavefront = p->integrator == CPT_INTEGRATOR_WAVEFRONT;
+    if (wavefront || !out->on_device) CPT_NEED(need_pool(s->ctx));
+    if (wavefront || !out->on_device || stats) CPT_NEED(need_host(s->ctx));
     size_t np = (size_t)W * H;
     float* rgb = out->rgb;
     uint8_t* rgba8 = out->rgba8;
@@ -1098,7 +1107,7 @@ CPT_EXPORT cpt_status cpt_render(cpt_scene* s, const cpt_render_params* p, const
     CPT_CUDA(cudaMemsetAsync(s->ray_counter, 0, sizeof(unsigned long long), stream));
     if (stats) CPT_CUDA(cudaEventRecord(e0, stream));
     cpt_status st = CPT_OK;
-    if (p->integrator == CPT_INTEGRATOR_WAVEFRONT) {
+    if (wavefront) {
         cpt_context* c = s->ctx;
         if (!c->wf_grids_ready) {
             st = wavefront_grids(c->sm_count, c->wf.block_trace, c->wf.block_shade, c->wf.short_stack, &c->wf.grid_trace, &c->wf.grid_trace_wide,

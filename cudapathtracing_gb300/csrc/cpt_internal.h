@@ -130,7 +130,8 @@ cpt_status launch_render_wavefront(const SceneView& view, const RenderArgs& args
 cpt_status launch_render_wavefront_batch(const SceneView* views, const RenderArgs* args, int n_jobs,
                                          cudaStream_t stream, const WavefrontTuning& tune);
 
-// The reference's joint-bilateral and temporal filters (filter.cu); device buffers.
+// The reference's joint-bilateral and temporal filters (filter.cu); device buffers.  pool: of the
+// bilateral filter's intermediate image, NULL: the device's default pool.
 DevCamera camera_of(const cpt_camera& c);
 cpt_status filter_bilateral(const float* rgb, const float* gbuf, float* out, int W, int H, const cpt_filter_params& p,
                             cudaStream_t stream, cudaMemPool_t pool);

@@ -368,7 +368,9 @@ cpt_status filter_bilateral(const float* rgb, const float* gbuf, float* out, int
     k.kd = 1.0f / (2.0f * p.sigma_d * p.sigma_d);
     k.radius = p.radius;
     float* tmp = nullptr;
-    CPT_CUDA(cudaMallocFromPoolAsync((void**)&tmp, (size_t)W * H * 3 * sizeof(float), pool, stream));
+    const size_t bytes = (size_t)W * H * 3 * sizeof(float);
+    if (pool) CPT_CUDA(cudaMallocFromPoolAsync((void**)&tmp, bytes, pool, stream));
+    else CPT_CUDA(cudaMallocAsync((void**)&tmp, bytes, stream));
     if (p.radius <= SMALL_RADIUS) {
         dim3 block(32, 8), grid((W + 31) / 32, (H + 7) / 8);
         k_bilateral_small<true><<<grid, block, 0, stream>>>(rgb, (const float4*)gbuf, tmp, W, H, k);
