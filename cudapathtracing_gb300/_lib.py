@@ -38,6 +38,7 @@ def lib():
             "cpt_last_error_string": (C.c_char_p, []),
             "cpt_context_create": (S, [C.c_int, C.POINTER(P)]),
             "cpt_context_destroy": (S, [P]),
+            "cpt_context_trim": (S, [P]),
             "cpt_context_set_render_block": (S, [P, C.c_int, C.c_int]),
             "cpt_context_set_wavefront": (S, [P, C.c_int, C.c_int, C.c_int, C.c_int]),
             "cpt_context_set_bvh_width": (S, [P, C.c_int]),

@@ -11,7 +11,7 @@ from dataclasses import dataclass, field
 import numpy as np
 
 # cpt_status
-CPT_OK = 0
+CPT_OK, CPT_ERR_INVALID_ARGUMENT, CPT_ERR_OUT_OF_MEMORY = 0, 1, 3
 STATUS_NAMES = {
     0: "CPT_OK",
     1: "CPT_ERR_INVALID_ARGUMENT",

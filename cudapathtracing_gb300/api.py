@@ -66,6 +66,10 @@ class Context:
     def set_short_stack(self, entries: int) -> None:
         check(lib().cpt_context_set_short_stack(self.h, entries), "cpt_context_set_short_stack")
 
+    def trim(self) -> None:
+        """Idle workspace memory back to the system (cpt_context_trim)."""
+        check(lib().cpt_context_trim(self.h), "cpt_context_trim")
+
     def close(self):
         if self.h:
             lib().cpt_context_destroy(self.h)

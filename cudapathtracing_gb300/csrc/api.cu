@@ -58,11 +58,7 @@ struct cpt_context {
     int bvh_width;             // traversal layout built by cpt_lbvh_build: 8 (compressed wide) or 2
     int iter_limit;            // loop trips per sample of the render loops (cpt_context_set_loop_limits)
     bool bvh2_compressed;      // BVH2 nodes of later builds: 32-byte quantised (cpt_context_set_bvh_compression)
-    // Workspaces of the calls (path slots, filter and host-image buffers) come from a pool of the
-    // context's own that keeps up to pool_keep bytes between calls and goes with the context.  The
-    // device's default pool gives everything back to the system whenever a stream is waited for, and
-    // every call waits: 0.33 ms per call for a 256 x 256 preview's slots, 0.2 ms for a 1080p filter.
-    cudaMemPool_t pool;        // NULL until need_pool
+    cudaMemPool_t pool;        // the device's workspace pool (workspace.cu), NULL until need_pool
     HostWords* host;           // pinned words that results are read back into, or NULL (need_host)
     char* staging;             // pinned and mapped: rays and hits of small host-memory queries, or NULL
     char* staging_dev;         // its device address
@@ -132,8 +128,7 @@ cpt_status dalloc(T** p, size_t count)
 {
     *p = nullptr;
     if (count == 0) return CPT_OK;
-    CPT_CUDA(cudaMalloc((void**)p, count * sizeof(T)));
-    return CPT_OK;
+    return device_alloc((void**)p, count * sizeof(T));
 }
 
 template <typename T>
@@ -449,26 +444,12 @@ SceneView view_of(const cpt_scene* s)
     return v;
 }
 
-// The context's workspace pool, made by the first call that needs it.
+// The workspace pool, taken by the first call that needs it.
 cpt_status need_pool(cpt_context* c)
 {
     if (c->pool) return CPT_OK;
-    cudaMemPoolProps props;
-    std::memset(&props, 0, sizeof props);
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = c->device;
-    size_t free_bytes = 0, total_bytes = 0;
-    CPT_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
-    uint64_t keep = total_bytes / 40;   // 7 GB of 284: the largest wavefront (16M slots) takes 5.4
-    cudaMemPool_t pool = nullptr;
-    CPT_CUDA(cudaMemPoolCreate(&pool, &props));
-    cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    if (e != cudaSuccess) {
-        cudaMemPoolDestroy(pool);
-        return cuda_fail(e, "workspace pool");
-    }
-    c->pool = c->wf.pool = pool;
+    CPT_NEED(pool_acquire(c->device, &c->pool));
+    c->wf.pool = c->pool;
     return CPT_OK;
 }
 
@@ -490,12 +471,6 @@ cpt_status need_host(cpt_context* c)
     c->wf.host_cnt = h->cnt;
     return CPT_OK;
 }
-
-#define CPT_NEED(call)                      \
-    do {                                    \
-        cpt_status _s = (call);             \
-        if (_s != CPT_OK) return _s;        \
-    } while (0)
 
 // Binary traversal nodes (either format), allocated on first use.
 cpt_status need_nodes(cpt_scene* s)
@@ -624,11 +599,18 @@ CPT_EXPORT cpt_status cpt_context_destroy(cpt_context* ctx)
             for (cudaEvent_t e : ctx->time) cudaEventDestroy(e);
             cudaFreeHost(ctx->host);
         }
-        if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
+        if (ctx->pool) pool_release(ctx->device);
         if (ctx->staging) cudaFreeHost(ctx->staging);
     }
     delete ctx;
     return CPT_OK;
+}
+
+CPT_EXPORT cpt_status cpt_context_trim(cpt_context* ctx)
+{
+    if (!ctx) return fail(CPT_ERR_INVALID_ARGUMENT, "cpt_context_trim: null context");
+    CPT_CUDA(cudaSetDevice(ctx->device));
+    return pool_trim(ctx->device);
 }
 
 // Internal tuning knob (the autotuner's setter): wavefront size, block sizes, graph replay.
@@ -1039,10 +1021,14 @@ CPT_EXPORT cpt_status cpt_trace_closest(cpt_scene* s, const cpt_ray* rays, uint6
     CPT_NEED(need_pool(c));
     cpt_ray* dr = nullptr;
     cpt_hit* dh = nullptr;
-    CPT_CUDA(cudaMallocFromPoolAsync((void**)&dr, n * sizeof(cpt_ray), c->pool, stream));
-    CPT_CUDA(cudaMallocFromPoolAsync((void**)&dh, n * sizeof(cpt_hit), c->pool, stream));
+    CPT_NEED(pool_alloc((void**)&dr, n * sizeof(cpt_ray), c->pool, stream));
+    cpt_status st = pool_alloc((void**)&dh, n * sizeof(cpt_hit), c->pool, stream);
+    if (st != CPT_OK) {
+        cudaFreeAsync(dr, stream);
+        return st;
+    }
     CPT_CUDA(cudaMemcpyAsync(dr, rays, n * sizeof(cpt_ray), cudaMemcpyHostToDevice, stream));
-    cpt_status st = launch_trace(v, dr, n, dh, s->err, stream, c->trace_resident);
+    st = launch_trace(v, dr, n, dh, s->err, stream, c->trace_resident);
     if (st == CPT_OK) CPT_CUDA(cudaMemcpyAsync(hits, dh, n * sizeof(cpt_hit), cudaMemcpyDeviceToHost, stream));
     cudaFreeAsync(dr, stream);
     cudaFreeAsync(dh, stream);
@@ -1081,11 +1067,16 @@ CPT_EXPORT cpt_status cpt_render(cpt_scene* s, const cpt_render_params* p, const
     float* gbuf = out->gbuffer;
     bool host = !out->on_device;
     if (host) {
-        CPT_CUDA(cudaMallocFromPoolAsync((void**)&rgb, np * 12, s->ctx->pool, stream));
+        cpt_status st = pool_alloc((void**)&rgb, np * 12, s->ctx->pool, stream);
+        if (st == CPT_OK && out->rgba8) st = pool_alloc((void**)&rgba8, np * 4, s->ctx->pool, stream);
+        if (st == CPT_OK && out->gbuffer) st = pool_alloc((void**)&gbuf, np * 32, s->ctx->pool, stream);
+        if (st != CPT_OK) {   // what was made has replaced the caller's pointer
+            if (rgba8 != out->rgba8) cudaFreeAsync(rgba8, stream);
+            if (rgb != out->rgb) cudaFreeAsync(rgb, stream);
+            return st;
+        }
         if (p->flags & CPT_RENDER_ACCUMULATE)
             CPT_CUDA(cudaMemcpyAsync(rgb, out->rgb, np * 12, cudaMemcpyHostToDevice, stream));
-        if (out->rgba8) CPT_CUDA(cudaMallocFromPoolAsync((void**)&rgba8, np * 4, s->ctx->pool, stream));
-        if (out->gbuffer) CPT_CUDA(cudaMallocFromPoolAsync((void**)&gbuf, np * 32, s->ctx->pool, stream));
     }
     RenderArgs a;
     a.spp = p->spp;
@@ -1210,10 +1201,12 @@ CPT_EXPORT cpt_status cpt_render_batch(cpt_context* ctx, const cpt_render_job* j
         if (!j.output.on_device) {   // device copies of host outputs for the duration of the call
             auto tmp = [&](auto** dst, size_t bytes, const void* init) {
                 void* d = nullptr;
-                cudaError_t e = cudaMallocFromPoolAsync(&d, bytes, ctx->pool, stream);
-                if (e == cudaSuccess && init) e = cudaMemcpyAsync(d, init, bytes, cudaMemcpyHostToDevice, stream);
+                st = pool_alloc(&d, bytes, ctx->pool, stream);
+                if (st != CPT_OK) return;
+                const cudaError_t e =
+                    init ? cudaMemcpyAsync(d, init, bytes, cudaMemcpyHostToDevice, stream) : cudaSuccess;
                 if (e != cudaSuccess) {
-                    if (d) cudaFreeAsync(d, stream);
+                    cudaFreeAsync(d, stream);
                     st = cuda_fail(e, "cpt_render_batch: device output");
                     return;
                 }

@@ -25,10 +25,23 @@ cpt_status cuda_fail(cudaError_t e, const char* what);
         if (_e != cudaSuccess) return ::cpt::cuda_fail(_e, #call); \
     } while (0)
 
+#define CPT_NEED(call)                      \
+    do {                                    \
+        cpt_status _s = (call);             \
+        if (_s != CPT_OK) return _s;        \
+    } while (0)
+
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // Count of kernels this library has launched since it was loaded (cpt_launch_count).
 void add_launches(uint64_t k);
+
+// ---- device memory (workspace.cu).  The current device's: every entry point has selected its context's.
+cpt_status pool_acquire(int device, cudaMemPool_t* out);   // the device's workspace pool, for one more context
+void pool_release(int device);
+cpt_status pool_trim(int device);                          // idle workspace back to the system
+cpt_status pool_alloc(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t stream);
+cpt_status device_alloc(void** p, size_t bytes);           // cudaMalloc
 
 // ---- LBVH build on caller-provided device buffers (lbvh.cu)
 struct LbvhBuffers {
@@ -119,7 +132,7 @@ struct WavefrontTuning {
     cudaStream_t capture_stream; // non-default stream used only to capture the iteration graph
     cudaStream_t side_stream;    // second stream: shadow rays traced beside extension rays
     cudaEvent_t fork, join;      // dependencies between the two streams
-    cudaMemPool_t pool;          // the context's workspace pool
+    cudaMemPool_t pool;          // the device's workspace pool
     int* host_cnt;               // pinned: the counters read back between chunks of iterations
 };
 

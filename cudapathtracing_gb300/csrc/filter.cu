@@ -369,7 +369,7 @@ cpt_status filter_bilateral(const float* rgb, const float* gbuf, float* out, int
     k.radius = p.radius;
     float* tmp = nullptr;
     const size_t bytes = (size_t)W * H * 3 * sizeof(float);
-    if (pool) CPT_CUDA(cudaMallocFromPoolAsync((void**)&tmp, bytes, pool, stream));
+    if (pool) CPT_NEED(pool_alloc((void**)&tmp, bytes, pool, stream));
     else CPT_CUDA(cudaMallocAsync((void**)&tmp, bytes, stream));
     if (p.radius <= SMALL_RADIUS) {
         dim3 block(32, 8), grid((W + 31) / 32, (H + 7) / 8);

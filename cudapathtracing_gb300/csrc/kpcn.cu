@@ -742,15 +742,15 @@ cpt_status net_init(Net& n, uint64_t seed)
             h[n.woff[i] + k] = (float)(stdv * std::sqrt(-2.0 * std::log(u1)) * std::cos(6.283185307179586 * u2));
         }
     }
-    CPT_CUDA(cudaMalloc((void**)&n.w, off * sizeof(float)));
-    CPT_CUDA(cudaMalloc((void**)&n.gw, off * sizeof(float)));
-    CPT_CUDA(cudaMalloc((void**)&n.m, off * sizeof(float)));
-    CPT_CUDA(cudaMalloc((void**)&n.v, off * sizeof(float)));
-    CPT_CUDA(cudaMalloc((void**)&n.wf16, o16 * sizeof(__nv_bfloat16)));
-    CPT_CUDA(cudaMalloc((void**)&n.wd16, o16 * sizeof(__nv_bfloat16)));
+    CPT_NEED(device_alloc((void**)&n.w, off * sizeof(float)));
+    CPT_NEED(device_alloc((void**)&n.gw, off * sizeof(float)));
+    CPT_NEED(device_alloc((void**)&n.m, off * sizeof(float)));
+    CPT_NEED(device_alloc((void**)&n.v, off * sizeof(float)));
+    CPT_NEED(device_alloc((void**)&n.wf16, o16 * sizeof(__nv_bfloat16)));
+    CPT_NEED(device_alloc((void**)&n.wd16, o16 * sizeof(__nv_bfloat16)));
     CPT_CUDA(cudaMemcpy(n.w, h.data(), off * sizeof(float), cudaMemcpyHostToDevice));
     CPT_CUDA(cudaDeviceGetAttribute(&n.sm_count, cudaDevAttrMultiProcessorCount, n.device));
-    CPT_CUDA(cudaMalloc((void**)&n.err, sizeof(int)));
+    CPT_NEED(device_alloc((void**)&n.err, sizeof(int)));
     CPT_CUDA(cudaMemset(n.err, 0, sizeof(int)));
     CPT_CUDA(cudaFuncSetAttribute(k_conv3x3_tc<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_MAX));
     CPT_CUDA(cudaFuncSetAttribute(k_conv3x3_tc<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_MAX));
@@ -846,7 +846,7 @@ cpt_status ensure_geometry(Net& n, int N, int H, int W)
     f32(&n.bpart, (long)WG_CHUNKS * 512);
     size_t total = 0;
     for (auto& r : reqs) total += align_up(r.bytes, 256);
-    CPT_CUDA(cudaMalloc((void**)&n.arena, total));
+    CPT_NEED(device_alloc((void**)&n.arena, total));
     n.arena_bytes = total;
     char* p = n.arena;
     for (auto& r : reqs) {

@@ -1030,7 +1030,7 @@ cpt_status run_wavefront(const SceneView& view, const RenderArgs& args, const st
     w.n_jobs = MULTI ? (int)J.size() : 0;
     size_t bytes = wf_bytes(M, L, n_parts, n_gs, tune.material_sort, w.n_jobs);
     char* base = nullptr;
-    CPT_CUDA(cudaMallocFromPoolAsync((void**)&base, bytes, tune.pool, stream));
+    CPT_NEED(pool_alloc((void**)&base, bytes, tune.pool, stream));
     char* p = base;
     size_t left = bytes;
     size_t ml = (size_t)M * L;

@@ -252,7 +252,33 @@ class GpuExecutor:
     def estimate(self, job) -> int:
         return job_bytes(self.descs[job.jid].num_triangles, job.size, job.spp)
 
+    def _with_room(self, fn):
+        """fn(), and once more with the library's and torch's idle memory given back when it ran out of
+        device memory: both keep some between jobs, outside the scheduler's budget."""
+        import torch
+        from . import abi
+        from ._lib import CptError
+        try:
+            return fn()
+        except torch.cuda.OutOfMemoryError:
+            pass
+        except CptError as e:
+            if e.status != abi.CPT_ERR_OUT_OF_MEMORY:
+                raise
+        # out of the except clause: the exception kept the failed pass's scenes and tensors alive
+        self.ctx[0].trim()   # the lanes' contexts share the device's pool
+        torch.cuda.empty_cache()
+        return fn()
+
     def run(self, job, lane) -> int:
+        return self._with_room(lambda: self._run(job, lane))
+
+    def run_batch(self, jobs, lane) -> int:
+        """The jobs' scenes uploaded and built on the lane's stream, one cpt_render_batch over all
+        of them (one wavefront), then each denoised; returns the batch's rays."""
+        return self._with_room(lambda: self._run_batch(jobs, lane))
+
+    def _run(self, job, lane) -> int:
         import torch
         from . import abi, api
         from .training import RENDER
@@ -270,10 +296,7 @@ class GpuExecutor:
             sc.close()
         return r["rays"]
 
-
-    def run_batch(self, jobs, lane) -> int:
-        """The jobs' scenes uploaded and built on the lane's stream, one cpt_render_batch over all
-        of them (one wavefront), then each denoised; returns the batch's rays."""
+    def _run_batch(self, jobs, lane) -> int:
         import torch
         from . import api
         from .training import RENDER

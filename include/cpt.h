@@ -232,6 +232,12 @@ const char* cpt_last_error_string(void);
  * without its fixed 2,000,000-object pool). */
 cpt_status cpt_context_create(int device, cpt_context** out);
 cpt_status cpt_context_destroy(cpt_context* ctx);
+/* Workspaces (path slots, filter and host-image buffers) come from one memory pool per device, which
+ * the contexts on it share.  Between calls it keeps up to 1/40 of the device's memory (7 GB of 284) and
+ * the last context's destruction gives it back; an allocation of this library that does not fit takes
+ * it first.  cpt_context_trim gives the memory of finished calls back at once, for a program's other
+ * users of the device. */
+cpt_status cpt_context_trim(cpt_context* ctx);
 
 /* Render tuning used by the autotuner: megakernel thread-block shape (bx*by a multiple of 32,
  * at most 512).  The defaults are 16 x 8. */
