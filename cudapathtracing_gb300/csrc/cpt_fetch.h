@@ -25,11 +25,7 @@ CPT_HD int spread_lanes(int n, int warps)
 // Whether a warp that took `count` items from `base` on has seen the end.
 CPT_HD bool fetch_ends(uint32_t base, int count, int n) { return base + (uint32_t)count >= (uint32_t)n; }
 
-// The rank-th of them, or -1 past the end.
-CPT_HD int fetched_item(uint32_t base, int rank, int n)
-{
-    const uint32_t r = base + (uint32_t)rank;
-    return r < (uint32_t)n ? (int)r : -1;
-}
+// Whether number r, counted from a warp's base, is an item.
+CPT_HD bool is_item(uint32_t r, int n) { return r < (uint32_t)n; }
 
 }  // namespace cpt

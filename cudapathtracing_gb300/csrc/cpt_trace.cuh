@@ -587,14 +587,14 @@ __device__ __forceinline__ uint32_t trace_items_walk(const Views& views, int n, 
             base = __shfl_sync(0xffffffffu, base, 0);
             if (fetch_ends(base, __popc(m), n)) exhausted = true;
             if (idle) {
-                const int r = fetched_item(base, __popc(m & lane_mask_lt()), n);
-                if (r >= 0) {
+                const uint32_t r = base + (uint32_t)__popc(m & lane_mask_lt());
+                if (is_item(r, n)) {
                     float3 o, d;
                     float tmn, tmx;
                     int skip = -1;
-                    load(r, o, d, tmn, tmx, skip, scene);
+                    item = (int)r;
+                    load(item, o, d, tmn, tmx, skip, scene);
                     w.start(o, d, tmn, tmx, skip);
-                    item = r;
                     rays++;
                 }
             }

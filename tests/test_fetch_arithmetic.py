@@ -28,10 +28,9 @@ static long long run(int n, int warps, uint32_t start)
             counter += 32;
             ended = fetch_ends(base, 32, n);
             for (int k = 0; k < 32; ++k) {
-                const int r = fetched_item(base, k, n);
-                if (r < -1 || r >= n) return -1;
-                if (r >= 0) {
-                    if ((uint32_t)r != base + (uint32_t)k) return -1;
+                const uint32_t r = base + (uint32_t)k;
+                if (is_item(r, n)) {
+                    if ((int)r < 0) return -1;
                     ++items;
                 } else if (!ended) return -1;
             }
