@@ -1092,8 +1092,27 @@ uint32_t sort_tile(uint32_t n) { return (uint32_t)sort_threads(n) * (sort_thread
 // Words of the sort's chains hold two flag bits beside a count of up to n.
 size_t chain_word(uint32_t n) { return n < 1u << 30 ? 4 : 8; }
 
+// Upper pyramid of a build: unions of 16, 64, 256, ... sorted leaf boxes, level after level to one box; at
+// least the three levels that k_tree writes.
+size_t upper_boxes(uint32_t n)
+{
+    size_t boxes = 0;
+    uint32_t m = (uint32_t)(((uint64_t)n + 15) / 16);
+    for (int l = 0;; ++l) {
+        boxes += m;
+        if (m <= 1 && l >= 2) return boxes;
+        m = (m + 3) / 4;
+    }
+}
+
+// code0 and box_unsorted live through a build.  The rest of the scratch holds one stage's arrays after
+// another's: the sort's, the tree's (which keep the cleared words: n_crossing is one of them), a refit's.
 struct ScratchLayout {
-    size_t code0, code1, val1, totals, tickets, state, sort_clear, box_unsorted, levels, total;
+    size_t code0, box_unsorted, total;
+    size_t totals, tickets, state, sort_clear;   // the sort's counters and chains, cleared together
+    size_t code1, val1;                          // the sort's second buffers
+    size_t gaps, crossing, up;                   // tree
+    size_t levels;                               // refit: the box pyramid
     uint32_t num_tiles;
     int level_count;   // pyramid levels above the leaves (0 for a single leaf)
 };
@@ -1102,32 +1121,38 @@ ScratchLayout layout_for(uint32_t n)
 {
     ScratchLayout L;
     std::memset(&L, 0, sizeof L);
-    size_t off = 0;
-    auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 256); return o; };
     const uint32_t tile = sort_tile(n);
     L.num_tiles = (uint32_t)(((uint64_t)n + tile - 1) / tile);
-    L.code0 = take((size_t)n * 4);
-    // The sort's second buffers and its chains are dead once the tree is built; a refit's box pyramid
-    // takes their place.
-    const size_t n4 = align_up((size_t)n * 4, 256);
-    const size_t totals = RS_PASSES * RS_BINS * 4;
-    L.sort_clear = totals + 256 + (size_t)RS_PASSES * L.num_tiles * RS_BINS * chain_word(n);
-    const size_t sort_bytes = 2 * n4 + L.sort_clear;
     size_t lv_boxes = 0;
     for (uint32_t m = n; m > 1;) {
         m = (uint32_t)(((uint64_t)m + 3) / 4);
         lv_boxes += m;
         L.level_count++;
     }
-    const size_t shared = take(std::max(sort_bytes, lv_boxes * 32));
-    L.code1 = shared;
-    L.val1 = shared + n4;
-    L.totals = shared + 2 * n4;   // totals, tickets and chains are cleared together
-    L.tickets = L.totals + totals;
-    L.state = L.tickets + 256;
-    L.levels = shared;
+    size_t off = 0, end = 0;
+    auto take = [&](size_t bytes) {
+        const size_t o = off;
+        off = align_up(off + bytes, 256);
+        end = std::max(end, off);
+        return o;
+    };
+    L.code0 = take((size_t)n * 4);
     L.box_unsorted = take((size_t)n * 32);
-    L.total = off;
+    const size_t stages = off;
+    L.totals = take(RS_PASSES * RS_BINS * 4);
+    L.tickets = take(256);
+    const size_t cleared = off;
+    L.state = take((size_t)RS_PASSES * L.num_tiles * RS_BINS * chain_word(n));
+    L.sort_clear = off - L.totals;
+    L.code1 = take((size_t)n * 4);
+    L.val1 = take((size_t)n * 4);
+    off = cleared;
+    L.gaps = take(n);
+    L.crossing = take((size_t)n * 4);
+    L.up = take(upper_boxes(n) * 32);
+    off = stages;
+    L.levels = take(lv_boxes * 32);
+    L.total = end;
     return L;
 }
 
@@ -1260,14 +1285,14 @@ cpt_status lbvh_build(uint32_t n_extra, const double* extra_centroid, const floa
     if (st != CPT_OK) return st;
     if (stages) CPT_CUDA(cudaEventRecord(stages[2], stream));
 
-    // Hierarchy, leaf and node boxes.  The sort's second buffers are free: code1 takes the list of
-    // crossing gaps, val1 the upper pyramid levels (8/3 bytes a primitive), the chains' room the gaps.
-    int8_t* gaps = (int8_t*)(base + SL.state);
+    // Hierarchy, leaf and node boxes.
+    int8_t* gaps = (int8_t*)(base + SL.gaps);
+    uint32_t* crossing = (uint32_t*)(base + SL.crossing);
     uint32_t* n_crossing = (uint32_t*)(base + SL.tickets) + RS_PASSES;
-    float4* up = (float4*)val1;
+    float4* up = (float4*)(base + SL.up);
     const unsigned tree_grid = blocks_for(n, TREE_THREADS), top_grid = std::min(blocks_for(n, 64), TOP_BLOCKS);
     const auto tree = out.nodes ? k_tree<true> : k_tree<false>;
-    tree<<<tree_grid, TREE_THREADS, 0, stream>>>(code0, val0, (int)n, box_unsorted, out.leaf_box, out.keys, gaps, code1,
+    tree<<<tree_grid, TREE_THREADS, 0, stream>>>(code0, val0, (int)n, box_unsorted, out.leaf_box, out.keys, gaps, crossing,
                                                  n_crossing, up, out.child, out.range, out.node_box, out.nodes);
     if (n > TREE_THREADS) {   // nodes reach across blocks: the rest of the pyramid, then those nodes
         const uint32_t n2 = (n + 15) / 16, n3 = (n2 + 3) / 4;
@@ -1292,7 +1317,7 @@ cpt_status lbvh_build(uint32_t n_extra, const double* extra_centroid, const floa
             m = top;
         }
         const auto rest = out.nodes ? k_tree_top<true> : k_tree_top<false>;
-        rest<<<top_grid, 64, 0, stream>>>(code0, val0, (int)n, code1, n_crossing, gaps, out.leaf_box, up, out.child,
+        rest<<<top_grid, 64, 0, stream>>>(code0, val0, (int)n, crossing, n_crossing, gaps, out.leaf_box, up, out.child,
                                           out.range, out.node_box, out.nodes);
         add_launches(1);
     }
