@@ -419,7 +419,13 @@ struct Chain {
 // 2,048 keys took 29 us a pass (every tile adds up the hundreds running beside it) against 23.
 //
 // FIRST: the values are the positions.
-constexpr int CHAIN_POLLS = 4096;
+#ifndef CPT_CHAIN_POLLS
+#define CPT_CHAIN_POLLS 4096
+#endif
+#ifndef CPT_CHAIN_WIDE_FROM
+#define CPT_CHAIN_WIDE_FROM (1u << 30)   // primitives; at least SORT_MEDIUM + 1
+#endif
+constexpr int CHAIN_POLLS = CPT_CHAIN_POLLS;
 constexpr int CHAIN_BATCH = 8;   // tiles a thread fetches at once
 
 template <int THREADS, int ITEMS, typename Word>
@@ -1090,7 +1096,8 @@ constexpr uint32_t SORT_SMALL = 1u << 15, SORT_MEDIUM = 1u << 19;
 int sort_threads(uint32_t n) { return n <= SORT_SMALL ? 256 : n <= SORT_MEDIUM ? 512 : 1024; }
 uint32_t sort_tile(uint32_t n) { return (uint32_t)sort_threads(n) * (sort_threads(n) == 256 ? 4u : 8u); }
 // Words of the sort's chains hold two flag bits beside a count of up to n.
-size_t chain_word(uint32_t n) { return n < 1u << 30 ? 4 : 8; }
+size_t chain_word(uint32_t n) { return n < CPT_CHAIN_WIDE_FROM ? 4 : 8; }
+static_assert(CPT_CHAIN_WIDE_FROM > SORT_MEDIUM && CPT_CHAIN_WIDE_FROM <= 1u << 30, "64-bit chains run on the largest tiles");
 
 // Upper pyramid of a build: unions of 16, 64, 256, ... sorted leaf boxes, level after level to one box; at
 // least the three levels that k_tree writes.
