@@ -43,10 +43,10 @@ struct BilateralConsts {
 // share a packed multiply-add.  The horizontal pass keeps its row, one array per component, in shared
 // memory (four neighbours' component in one conflict-free 16-byte load); in the vertical pass lanes
 // are neighbouring columns and read the images directly.  Each pixel's taps are added in the
-// window's order, and its multiply-adds are those of the pixel-a-thread form, so both give the same
-// bits.  Both passes, radius 16 at 1920x1080: 227 us with a pixel a thread, 174 us so.  Other forms of
-// this one: scalar multiply-adds +19 us, 80 registers (three blocks an SM) +20, distances from
-// converted tap numbers instead of a table +4; the exponentials are 27 us of it.
+// window's order, with the multiply-adds that the compiler forms for a pixel a thread, so both give the
+// same bits (tests/test_gpu_filter_forms.py).  Both passes, radius 16 at 1920x1080: 227 us with a pixel a
+// thread, 174 us so.  Other forms of this one: scalar multiply-adds +19 us, 80 registers (three blocks an
+// SM) +20, distances from converted tap numbers instead of a table +4; the exponentials are 27 us of it.
 constexpr int FPX = 4;   // pixels a thread; also neighbours a step
 
 __device__ __forceinline__ uint64_t pack2(float a, float b)
@@ -264,7 +264,10 @@ __global__ void __launch_bounds__(32 * VROWS, 2) k_bilateral_columns(const float
 // wider form's staging and unfilled steps cost more than they save (us at 1920x1080, 901x507 and
 // 100x400; a pixel a thread / four: radius 4 82 / 92, 30 / 36, 16 / 18; 6 106 / 105, 37 / 39, 16 / 20;
 // 8 129 / 116, 45 / 43, 19 / 20; 16 227 / 174, 69 / 61, 26 / 24).
-constexpr int SMALL_RADIUS = 6;
+#ifndef CPT_FILTER_SMALL_RADIUS
+#define CPT_FILTER_SMALL_RADIUS 6
+#endif
+constexpr int SMALL_RADIUS = CPT_FILTER_SMALL_RADIUS;
 
 template <bool HORIZONTAL>
 __global__ void __launch_bounds__(256) k_bilateral_small(const float* __restrict__ src, const float4* __restrict__ gbuf,
@@ -376,7 +379,7 @@ cpt_status filter_bilateral(const float* rgb, const float* gbuf, float* out, int
         k_bilateral_small<true><<<grid, block, 0, stream>>>(rgb, (const float4*)gbuf, tmp, W, H, k);
         k_bilateral_small<false><<<grid, block, 0, stream>>>(tmp, (const float4*)gbuf, out, W, H, k);
     } else {
-        // rows a block: as many as the default 48 KB of shared memory hold (8 up to radius 38, 2 at 256)
+        // rows a block: as many as the default 48 KB of shared memory hold (8 up to radius 44, 2 at 256)
         const size_t table = sizeof(float2) * table_size(p.radius), row = 7 * sizeof(float) * h_pitch(p.radius);
         const int rows = (int)std::min<size_t>(8, (48 * 1024 - table) / row);
         k_bilateral_rows<<<dim3((unsigned)((W + HTILE - 1) / HTILE) * ((H + rows - 1) / rows)), dim3(32, rows), table + rows * row, stream>>>(
