@@ -753,7 +753,8 @@ __global__ void __launch_bounds__(256, 4) k_wf_shade(const __grid_constant__ Sce
 //
 // Rays are advanced one node per trip, as in the trace kernels; a lane whose ray is done waits
 // until 1 / PATHS_SHARE of its warp's busy lanes do before it shades and starts its next ray, so the
-// divergent shading code runs for several lanes at a time.  Few slots are spread over all warps.  The
+// divergent shading code runs for several lanes at a time.  Fewer slots than the launch has lanes (the last
+// paths of a large render; a small render's launch has a lane a slot) are spread over its warps.  The
 // slot's state stays where the queue kernels keep it and both run the same shade_vertex, so a
 // render may change over between iterations and its image does not depend on when it does.
 //
@@ -962,8 +963,15 @@ namespace {
 // several times over, single samples keep more slots busy and end sooner (a batch of six small
 // renders, 1.77M groups: 28.3 -> 20.6 ms; a 256 x 256, 4-spp frame, 65K groups: 4.7 -> 2.3 ms), and
 // where they do, starting an item costs more than it gives (64-spp 1080p, 16.6M groups: 281 -> 300
-// ms).  The second bound keeps the per-sample sums (16 bytes, with a G-buffer 48) under 1 GB.
-bool single_samples(size_t groups, size_t samples) { return groups <= (size_t)1 << 21 && samples <= (size_t)1 << 24; }
+// ms).  Several times is 8: 1024 x 1024 at 8 and 16 spp with groups / single samples, 65,536 slots
+// (16 and 32 times) 92 / 97 and 184 / 193 ms, 131,072 (8 and 16) 55 / 57 and 110 / 113, 262,144 (4 and
+// 8) 46 / 43 and 92 / 86.  A render that k_wf_paths runs alone always takes single samples.  The bound on
+// samples keeps their sums (16 bytes, with a G-buffer 48) under 1 GB.
+bool single_samples(size_t groups, size_t samples, size_t slots)
+{
+    return samples <= (size_t)PATHS_SLOTS ||
+           (groups <= (size_t)1 << 21 && groups <= 8 * slots && samples <= (size_t)1 << 24);
+}
 
 // A single render (jobs empty: scene and parameters in kernel arguments) or a batch (MULTI).
 template <bool MULTI>
@@ -972,6 +980,7 @@ cpt_status run_wavefront(const SceneView& view, const RenderArgs& args, const st
 {
     Wf w;
     std::memset(&w, 0, sizeof w);
+    const size_t slots = (size_t)std::max(tune.slots, 1024);
     size_t n_items = 0, n_parts = 0, n_gs = 0;
     int L = 1;
     std::vector<WfJob> J = jobs;
@@ -985,7 +994,7 @@ cpt_status run_wavefront(const SceneView& view, const RenderArgs& args, const st
         if (args.spp <= 0) return fail(CPT_ERR_INVALID_ARGUMENT, "spp must be positive");
         w.SG = sample_group(args.spp);
         const size_t groups = (size_t)((args.spp + w.SG - 1) / w.SG) * (size_t)w.npix;
-        w.S = single_samples(groups, (size_t)args.spp * (size_t)w.npix) ? 1 : w.SG;
+        w.S = single_samples(groups, (size_t)args.spp * (size_t)w.npix, slots) ? 1 : w.SG;
         n_items = n_parts = (size_t)((args.spp + w.S - 1) / w.S) * (size_t)w.npix;
         if (w.S != w.SG && args.gbuf) n_gs = 2 * (size_t)std::min(w.SG, args.spp) * (size_t)w.npix;
         L = std::max(view.n_lights, 1);
@@ -1002,7 +1011,7 @@ cpt_status run_wavefront(const SceneView& view, const RenderArgs& args, const st
             samples += (size_t)j.args.spp * (size_t)std::max(j.npix, 0);
         }
         for (WfJob& j : J) {
-            j.S = single_samples(groups, samples) ? 1 : j.SG;
+            j.S = single_samples(groups, samples, slots) ? 1 : j.SG;
             j.gs_base = -1;
             if (j.S != j.SG && j.args.gbuf) {
                 j.gs_base = (long long)n_gs;
@@ -1021,7 +1030,7 @@ cpt_status run_wavefront(const SceneView& view, const RenderArgs& args, const st
         if (n_items == 0) return CPT_OK;
     }
     if (n_items > (size_t)INT32_MAX / 2) return fail(CPT_ERR_UNSUPPORTED, "wavefront integrator: too many pixel groups");
-    const int M = (int)std::min(n_items, (size_t)std::max(tune.slots, 1024));
+    const int M = (int)std::min(n_items, slots);
     w.M = M;
     w.L = L;
     w.n_items = (int)n_items;
