@@ -10,9 +10,13 @@ LBVH build over the resident triangles + the full 64-spp render.  Synthetic, see
              shapes from the autotuner, timed (untimed here) at the workload's own spp up to 64
   e2e        same metric through the C ABI with host buffers: scene upload from pinned host
              memory, build, render, image read-back, scene release — every step
-  roofline   the render kernel: algorithmic bytes per ray (oracle-counted traversal work of the
-             workload, cudapathtracing_gb300/workload_constants.json) x rays / kernel time;
-             traffic = measured DRAM bytes per traced ray (profiles/traffic_<workload>.json) x rays
+  roofline   the render against the measured copy bandwidth: achieved = DRAM bytes per traced ray from
+             an ncu pass over every launch of one render (profiles/traffic_<workload>.json) x rays /
+             device time.  The traversal kernels are bound by issue slots, the integer pipe and
+             dependent loads, not by DRAM.  Beside it the bytes per ray that an ordered, pruned walk
+             of the binary tree reads (oracle-counted, cudapathtracing_gb300/workload_constants.json):
+             most of them come from L2, so their rate may exceed the DRAM peak.  Without a traffic
+             file (the trace workload) achieved and frac are null.
   cpu_baseline  the reference's bounce loop on the host cores with the workload's own estimator
              and spp on a band of rows (the oracle's FP64 restatement; oracle/_ref, the reference's
              own code, for its STATIC estimator where built), plus the STATIC estimator at 1 spp
@@ -582,9 +586,9 @@ def main():
         peak, peak_src = 6800.0, "fallback"
     k_ms = float(np.mean(kernel_ms))
     rays_per_launch = rays / world / args.steps
-    achieved = rays_per_launch * bpr / (k_ms / 1e3) / 1e9
+    model_gbs = rays_per_launch * bpr / (k_ms / 1e3) / 1e9
     # DRAM bytes per launch from the committed ncu capture: measured bytes per traced ray of the
-    # integrator (every launch of a 2-spp render, one-pass metrics) times this run's rays per launch
+    # integrator (every launch of a render, one-pass metrics) times this run's rays per launch
     traffic = None
     tpath = os.path.join(ROOT, "profiles", f"traffic_{args.workload}.json")
     if os.path.exists(tpath):
@@ -594,6 +598,7 @@ def main():
             traffic = int(src["bytes_per_ray"] * rays_per_launch)
         else:
             traffic = src.get("bytes_per_launch")
+    achieved = traffic / (k_ms / 1e3) / 1e9 if traffic else None
 
     # second half of the metric: wall time to display-space RMSE 0.01, denoised vs plain spp
     denoise = None
@@ -645,11 +650,13 @@ def main():
                               "probe_default_mrays": round(tuned.default_score, 1)} if tuned else None)},
         "e2e": {"value": round(e2e_rays / e2e_t / 1e6, 3), "unit": "Mrays/s", "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h), "steps": e2e_steps},
-        "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-                     "frac": round(achieved / peak, 4), "traffic": traffic,
+        "roofline": {"bound": "issue slots and dependent loads (traversal), DRAM (shading)",
+                     "achieved": round(achieved, 1) if achieved else None, "peak": peak, "unit": "GB/s",
+                     "frac": round(achieved / peak, 4) if achieved else None, "traffic": traffic,
                      "kernel": "k_trace_dyn" if trace_only else (
                          "k_wf_* (every launch of one render)" if args.integrator == "wavefront" else "k_render"),
-                     "kernel_ms": round(k_ms, 3), "bytes_per_ray": round(bpr, 1), "peak_source": peak_src},
+                     "kernel_ms": round(k_ms, 3), "peak_source": peak_src,
+                     "binary_walk": {"bytes_per_ray": round(bpr, 1), "gbs": round(model_gbs, 1)}},
         "cpu_baseline": cpu,
         "cpu_sample_on_gpu": same_gpu,
         "megakernel_same_run": compare,

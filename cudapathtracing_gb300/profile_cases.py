@@ -1,7 +1,7 @@
 """Small, self-contained invocations of each kernel family, sized for per-kernel ncu captures
 (a few hundred MB on the device, a handful of launches of the kernel of interest).
 
-    python -m cudapathtracing_gb300.profile_cases render  [--integrator wavefront|megakernel] [--layout bvh2|bvh2q|bvh8]
+    python -m cudapathtracing_gb300.profile_cases render  [--integrator wavefront|megakernel] [--layout bvh2|bvh2q|bvh8] [--slots N]
     python -m cudapathtracing_gb300.profile_cases trace   [--layout ...] [--rays N]
     python -m cudapathtracing_gb300.profile_cases build   [--layout ...]
     python -m cudapathtracing_gb300.profile_cases filter
@@ -42,10 +42,12 @@ def main(argv=None) -> None:
     ap.add_argument("--integrator", default="wavefront", choices=["wavefront", "megakernel"])
     ap.add_argument("--spp", type=int, default=1)
     ap.add_argument("--frames", type=int, default=2)
+    ap.add_argument("--slots", type=int, default=1 << 21, help="path slots of the wavefront")
     ap.add_argument("--rays", type=int, default=2_000_000)
     a = ap.parse_args(argv)
     import torch
     ctx = _context(a.layout)
+    ctx.set_wavefront(a.slots)
     if a.case == "render":
         s = api.Scene(ctx, P.spheres_scene()).init()
         rgb = torch.zeros((s.height, s.width, 3), device="cuda")
