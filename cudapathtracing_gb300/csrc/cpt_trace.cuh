@@ -141,8 +141,8 @@ __device__ __forceinline__ float3 safe_inverse(float3 d)
 }
 
 // 32 bytes of read-only memory (32-byte aligned) in one load: the traversals are divergent, so each
-// load is an L1 request of its own lines per lane (10M queries through the 64-byte BVH2 nodes of a
-// 1.31M-triangle mesh: 1.626 ms with four 16-byte loads a node, 1.595 ms with two of these).
+// load is an L1 request of its own lines per lane (the 64-byte BVH2 nodes take two of these in place of
+// four 16-byte loads: 10M queries of a 1.31M-triangle mesh 2 % faster at best, which runs differ by too).
 __device__ __forceinline__ void ldg8(const float4* p, float4& a, float4& b)
 {
     asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -204,8 +204,8 @@ __device__ __forceinline__ uint32_t xor_bits(uint32_t v, uint32_t o)
 // warp can refill finished lanes (dynamic fetching); Stack64 keeps group entries (in shared and
 // local memory, or local only).
 //
-// The walk is bound by issue slots and the integer/min-max pipe (65 % and 53 % busy with 17 of 32
-// lanes active, against 3 % of DRAM), so a visit is written for few such instructions: planes are
+// The walk is bound by issue slots and the integer/min-max pipe (58-62 % and 52-57 % busy with 17 to 20
+// of 32 lanes active, against 5 % of DRAM; before this visit 65-69 % of the issue slots), so a visit is written for few such instructions: planes are
 // taken in the ray's order (no min/max per plane pair), bytes become floats by one permute, two
 // children share a packed multiply-add, three-input min/max, and a miss is the sign bit of the
 // interval's length shifted into a mask.  On the 64-spp 1080p frame of 4.1M triangles: 365 ms with

@@ -1089,9 +1089,16 @@ __global__ void k_leaf_records(const uint32_t* __restrict__ order, uint32_t n, u
 
 inline unsigned blocks_for(uint64_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
 
-// Threads of a sort block (4 or 8 keys each).  A tile adds up the counts of the tiles before it that
-// run beside it, so there should be about as many tiles as SMs; below that, small tiles, since a pass
-// lasts as long as one tile.
+// Threads of a sort block (4 or 8 keys each).  A tile adds up the counts of the tiles before it that run
+// beside it, so large sorts want about as many tiles as SMs; below that, small tiles, since a pass lasts
+// as long as one tile.  Whole builds (us) with blocks of 256 / 512 / 1,024 threads at every size:
+//   32,768 73 / 76 / 92     196,608 104 / 105 / 115    655,360  167 / 152 / 150
+//   65,536 79 / 81 / 97     262,144 112 / 109 / 120  1,048,576  221 / 190 / 180
+//  131,072 89 / 95 / 107    524,288 150 / 130 / 140  1,310,720  258 / 212 / 219
+// The upper line lies between the middle shape's last size and the large one's first; at 1.31M the large
+// shape has 160 tiles for 152 SMs, and the last eight cost it its lead.  The lower line could be near
+// 200,000 (6 % of a build between) but for cpt_lbvh_build_device_static: with tiles of 1,024 keys the
+// chains of 65,536 primitives do not fit its 3 MiB.
 constexpr uint32_t SORT_SMALL = 1u << 15, SORT_MEDIUM = 1u << 19;
 int sort_threads(uint32_t n) { return n <= SORT_SMALL ? 256 : n <= SORT_MEDIUM ? 512 : 1024; }
 uint32_t sort_tile(uint32_t n) { return (uint32_t)sort_threads(n) * (sort_threads(n) == 256 ? 4u : 8u); }

@@ -34,8 +34,8 @@
 // the material its ray hit (miss / light / medium boundary, diffuse-like surfaces with next-event
 // estimation, specular dielectrics, rough dielectrics) and k_wf_shade walks the bins in order, so
 // the lanes of a warp run the same BSDF code.  A slot's result does not depend on the order in which
-// slots are shaded (its random numbers come from its own sample stream), so the image is the same.  The host replays a CUDA graph of CHUNK iterations and reads
-// the queue sizes after each replay to stop.
+// slots are shaded (its random numbers come from its own sample stream), so the image is the same.
+// The host replays a CUDA graph of CHUNK iterations and reads the queue sizes after each replay to stop.
 #include <cooperative_groups.h>
 #include <cooperative_groups/reduce.h>
 #include <cuda_runtime.h>

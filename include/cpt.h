@@ -156,9 +156,9 @@ typedef struct cpt_bvh_stats {
     uint32_t reserved;
     float ms_prep;       /* centroids, leaf boxes and Morton keys */
     float ms_sort;
-    float ms_emit;       /* Karras hierarchy emission */
-    float ms_refit;
-    float ms_collapse;   /* traversal layout */
+    float ms_emit;       /* a build's Karras hierarchy with its boxes and, for 64-byte nodes, the nodes */
+    float ms_refit;      /* a refit's whole time; about 0 for a build (its boxes come with the hierarchy) */
+    float ms_collapse;   /* traversal layout (what the hierarchy has not written) */
     float ms_total;
 } cpt_bvh_stats;
 
