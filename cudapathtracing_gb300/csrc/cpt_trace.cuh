@@ -253,11 +253,9 @@ struct WideWalk {
     // p - o, the product, c, the offset and the final multiply-add round by up to 2^-24 of (p - o) * idir,
     // c or t, of which the first two are at most |t| + 1.01 |A|.  So the near offset is moved down and the
     // far offset up by 2^-22 |A| = 2^-7 |a| (under 1 % of a grid step), and a distance is then at most
-    // 5 x 2^-24 |t| inside the exact one; NEAR_SLACK covers that where near and far are compared.  A ray
-    // that meets the stored box thus passes the test, for an origin at any distance.  (The slack on the
-    // far distance, or added to the offsets, costs: megakernel over this layout +1 to 2 %, more spilled
-    // registers; the 64-spp 1080p frame +2 %.)
-    static constexpr float NEAR_SLACK = 1.0f - 0x1p-20f;
+    // 5 x 2^-24 |t| inside the exact one; FAR_SLACK covers that where near and far are compared.  A ray
+    // that meets the stored box thus passes the test, for an origin at any distance.
+    static constexpr float FAR_SLACK = 1.0f + 0x1p-20f;
     __device__ __forceinline__ static void axis(float p, float o, float scale, float idir, float& A, float& bn, float& bf)
     {
         A = scale * idir * 32768.0f;
@@ -305,7 +303,7 @@ struct WideWalk {
             const float tn = fmaxf(max3f(nx[i], ny[i], nz[i]), tmin);                             \
             const float tf = fminf(min3f(fx[i], fy[i], fz[i]), best);                             \
             /* sign set: a miss */                                                                \
-            misses = __funnelshift_l(__float_as_uint(__fmaf_rn(tn, -NEAR_SLACK, tf)), misses, 1); \
+            misses = __funnelshift_l(__float_as_uint(__fmaf_rn(tf, FAR_SLACK, -tn)), misses, 1);  \
         }                                                                                         \
     }
             CPT_WIDE_PAIR(0)

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 f, d = np.float32, np.float64
-NEAR_SLACK = f(1 - 2.0 ** -20)
+FAR_SLACK = f(1 + 2.0 ** -20)
 
 
 def _fma(a, b, c):
@@ -50,7 +50,7 @@ def test_rays_that_meet_a_stored_box_pass(extent, fused):
     meets = (enter <= leave) & (leave >= 0.001)
     near, far = _planes(p, o, scale, idir, q, fused)
     tn, tf = np.maximum(near.max(1), f(0.001)), far.min(1)
-    passes = ~np.signbit(_fma(tn, np.full_like(tn, -NEAR_SLACK), tf))
+    passes = ~np.signbit(_fma(tf, np.full_like(tf, FAR_SLACK), -tn))
     assert meets.sum() > m // 20
     assert (passes | ~meets).all()
     # and little more: what passes comes within a grid step and the slack of the box
