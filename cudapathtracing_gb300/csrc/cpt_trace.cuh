@@ -249,13 +249,9 @@ struct WideWalk {
 
     // Slab distances along one axis as multiplier and offsets for byte_float values.  A byte q
     // stands for the plane p + q * scale at t = (p - o) * idir + q * a with a = scale * idir; with
-    // byte_float(q) = 1 + q * 2^-15 that is byte_float(q) * A + c with A = 2^15 a, c = (p - o) * idir - A.
-    // p - o, the product, c, the offset and the final multiply-add round by up to 2^-24 of (p - o) * idir,
-    // c or t, of which the first two are at most |t| + 1.01 |A|.  So the near offset is moved down and the
-    // far offset up by 2^-22 |A| = 2^-7 |a| (under 1 % of a grid step), and a distance is then at most
-    // 5 x 2^-24 |t| inside the exact one; FAR_SLACK covers that where near and far are compared.  A ray
-    // that meets the stored box thus passes the test, for an origin at any distance.
-    static constexpr float FAR_SLACK = 1.0f + 0x1p-20f;
+    // byte_float(q) = 1 + q * 2^-15 that is byte_float(q) * A + (b - A), A = 2^15 a.  b - A is
+    // rounded to half a unit of 2^-24 |A| = 2^-9 |a|, so the near offset is moved down and the far
+    // offset up by 2^-7 |a| (under 1 % of a grid step): the tested box contains the stored one.
     __device__ __forceinline__ static void axis(float p, float o, float scale, float idir, float& A, float& bn, float& bf)
     {
         A = scale * idir * 32768.0f;
@@ -302,8 +298,7 @@ struct WideWalk {
         {                                                                                         \
             const float tn = fmaxf(max3f(nx[i], ny[i], nz[i]), tmin);                             \
             const float tf = fminf(min3f(fx[i], fy[i], fz[i]), best);                             \
-            /* sign set: a miss */                                                                \
-            misses = __funnelshift_l(__float_as_uint(__fmaf_rn(tf, FAR_SLACK, -tn)), misses, 1);  \
+            misses = __funnelshift_l(__float_as_uint(tf - tn), misses, 1); /* sign set: a miss */ \
         }                                                                                         \
     }
             CPT_WIDE_PAIR(0)
