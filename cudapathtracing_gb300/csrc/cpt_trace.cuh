@@ -249,9 +249,14 @@ struct WideWalk {
 
     // Slab distances along one axis as multiplier and offsets for byte_float values.  A byte q
     // stands for the plane p + q * scale at t = (p - o) * idir + q * a with a = scale * idir; with
-    // byte_float(q) = 1 + q * 2^-15 that is byte_float(q) * A + (b - A), A = 2^15 a.  b - A is
-    // rounded to half a unit of 2^-24 |A| = 2^-9 |a|, so the near offset is moved down and the far
-    // offset up by 2^-7 |a| (under 1 % of a grid step): the tested box contains the stored one.
+    // byte_float(q) = 1 + q * 2^-15 that is byte_float(q) * A + (b - A), A = 2^15 a, b = (p - o) * idir.
+    // b - A is rounded to half a unit of 2^-24 |b - A|, 2^-9 |a| while |b| is not above |A|, so the near
+    // offset is moved down and the far offset up by 2^-7 |a| (under 1 % of a grid step): for origins within
+    // 2^17 grid steps of the node the tested box contains the stored one but for the roundings of b and of
+    // the final multiply-add, which every slab test has.  Farther out b - A adds one such rounding more,
+    // and a grazing ray may miss the box by it.  That is left so: with a slack of 2^-20 on the distances no
+    // ray misses, but rays from 30,000 units away then report hits of spheres (their boxes are not padded)
+    // that only the FP32 sphere test sees, which the binary layout does not report.
     __device__ __forceinline__ static void axis(float p, float o, float scale, float idir, float& A, float& bn, float& bf)
     {
         A = scale * idir * 32768.0f;
